@@ -34,6 +34,12 @@ struct mcb_heat_state {
   mcb::StreamMaps *maps = nullptr;
   uint8_t *code = nullptr;
   uint8_t *uniX = nullptr, *uniY = nullptr, *uniZ = nullptr;  // homogeneous-chunk tables (streamed)
+  // coded-row passes (heat_rows.cu): row codes per direction, their tables and hash keys
+  uint8_t *rowYZ = nullptr, *rowZMed = nullptr;
+  uint4 *rowX = nullptr, *rowY = nullptr, *rowZ = nullptr;
+  float4 *rowTab = nullptr;
+  unsigned long long *rowKeys = nullptr;
+  int *rowMed = nullptr;
   float *H = nullptr;
   float4 *Hd = nullptr;
   int codeHs = -1;
@@ -98,7 +104,7 @@ void stream_stepper_launch(const StreamStepper *k, cudaStream_t st);
 StreamShape stream_shape(int nx, int ny, int nz);
 int stream_warmup(const float *c, float hdt, int nM);
 void stream_carve(const std::function<void *(size_t)> &take, mcb_heat_state *s, const mcb_heat_params *p, bool damage,
-                  bool withQ);
+                  bool withQ, bool withRows);
 mcb_status stream_maps(mcb_ctx *ctx, mcb_heat_state *s);
 mcb_status stream_upload(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *p, const float *T, const float *Omega);
 mcb_status stream_upload_q(mcb_ctx *ctx, mcb_heat_state *s, const float *Q);
@@ -109,6 +115,13 @@ mcb_status stream_download(mcb_ctx *ctx, mcb_heat_state *s, float *T, float *Ome
 // asynchronous.
 void stream_dense_copy(mcb_ctx *ctx, const mcb_heat_state *s, float *dense, cudaStream_t st);
 void stream_dense_set(mcb_ctx *ctx, mcb_heat_state *s, const float *dense, cudaStream_t st);
+// Coded-row passes (heat_rows.cu): grids they take, the buffers of their row codes, the per-call
+// codes (*ok false: more row coefficients than the tables hold), and one step.
+struct StreamDev;
+bool rows_supported(int nx, int ny, int nz);
+void rows_carve(const std::function<void *(size_t)> &take, mcb_heat_state *s);
+mcb_status rows_build(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *p, bool *ok);
+void rows_step_launch(const mcb_heat_state *s, const StreamDev &h, cudaStream_t q);
 // Index of voxel v (dense, column-major) in a streamed state's pitched grids.
 long long stream_pitched_index(const mcb_heat_state *s, long long v);
 

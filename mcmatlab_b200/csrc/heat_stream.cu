@@ -1,6 +1,10 @@
 // Streamed DG-ADI stepper for sm_100a: the forward heat path of mcb_heat_forward and
 // mcb_heat_state_* (replacing +MCmatlab/src/finiteElementHeatPropagator.c:688-821) for grids
-// whose axes are at most 512 voxels long.
+// whose axes are at most 512 voxels long: state, set-up and host side, and the TMA-staged passes.
+// Calls step with the coded-row passes of heat_rows.cu where their row codes fit (2.0x the
+// TMA-staged passes at 100^3, 1.85x at 300x300x200); the TMA-staged passes step the others: media
+// that vary voxel by voxel (more than 255 row coefficients along an axis), calls of
+// mcb_heat_forward_static whose scratch has no room for the codes, and the adjoint's forward sweeps.
 //
 // One time step of the reference is six grid passes (substep1a..3b, :249-647). Here it is three
 // streaming passes, one per direction, and nothing per voxel is stored besides the state:
@@ -41,6 +45,7 @@
 #include <vector>
 
 #include "heat_host.h"
+#include "heat_stream.cuh"
 #include "tma.cuh"
 
 namespace mcb {
@@ -102,31 +107,6 @@ __device__ __forceinline__ int swz(int i, int j) { return i * 64 + ((((j >> 2) ^
 
 }  // namespace
 
-struct StreamDev {
-  int nx, ny, nz, nM, px, W;
-  long long sxy;  // px * ny
-  float *T, *A;
-  const uint8_t *M, *code;
-  const float *Q;     // or nullptr (light off)
-  float *dOmega;      // or nullptr
-  const float *H;     // [3][nM][nM]: H[d*nM*nM + mj*nM + mi] = dt/2 c(mi, mj, d)
-  const float4 *Hd;   // [nM] diagonal {H(m,m,0), H(m,m,1), H(m,m,2), 0}
-  const float4 *Hs;   // [nM] 1 / b*(m, d): inverse fixed-point pivot of a line of medium m along d
-  const float2 *dmg;  // [nM] Arrhenius exponent about the base temperature
-  float T0, dt;
-  unsigned int *maxEnc;
-  int hs;
-  double base;
-  int nS;
-  const double *sIdx, *sW;
-  double *sens;
-  int *stepCounter;
-  int *err;
-  // per-call tables of the homogeneous lane chunks (medium + 1, or 0): X pass [nz][ny][lanes],
-  // column-layout Y and Z passes [nOther][chunks][px] (stream_setup)
-  const uint8_t *uniX, *uniY, *uniZ;
-};
-
 namespace {
 
 // First 1024-byte boundary at or after p in shared memory (the swizzle pattern of the Y/Z tiles
@@ -148,23 +128,6 @@ __device__ __forceinline__ float frcp(float x) {
 
 __device__ __forceinline__ float hcoef(const StreamDev &h, int d, int mi, int mj) {
   return __ldg(h.H + (d * h.nM + mj) * h.nM + mi);
-}
-
-// Sensor interpolation (recordTempSensors, finiteElementHeatPropagator.c:652-664) on the pitched
-// state; sensor corner indices are dense 0-based linear indices.
-__device__ void record_sensors_p(const StreamDev &h, int col) {
-  for (int j = threadIdx.x; j < h.nS; j += blockDim.x) {
-    const long long li = (long long)h.sIdx[j];
-    const long long nxy = (long long)h.nx * h.ny;
-    const long long iz = li / nxy, r = li - iz * nxy, iy = r / h.nx, ix = r - iy * h.nx;
-    const long long i = ix + iy * h.px + iz * h.sxy, sx = 1, sy = h.px, sz = h.sxy;
-    const double wx = h.sW[j], wy = h.sW[j + h.nS], wz = h.sW[j + 2 * h.nS];
-    auto T = [&](long long k) { return (double)h.T[k] + h.base; };
-    h.sens[j + (long long)col * h.nS] =
-        (1 - wx) * (1 - wy) * (1 - wz) * T(i) + (1 - wx) * (1 - wy) * wz * T(i + sz) + (1 - wx) * wy * (1 - wz) * T(i + sy) +
-        (1 - wx) * wy * wz * T(i + sy + sz) + wx * (1 - wy) * (1 - wz) * T(i + sx) + wx * (1 - wy) * wz * T(i + sx + sz) +
-        wx * wy * (1 - wz) * T(i + sx + sy) + wx * wy * wz * T(i + sx + sy + sz);
-  }
 }
 
 // Pivots of a lane's `count` rows from their coefficients a[k], c[k] (rows s+k), given the
@@ -1251,7 +1214,7 @@ mcb_status stream_maps(mcb_ctx *ctx, mcb_heat_state *s) {
 
 // Buffers of the streamed state, carved by `take` (256-byte aligned pieces).
 void stream_carve(const std::function<void *(size_t)> &take, mcb_heat_state *s, const mcb_heat_params *p, bool damage,
-                  bool withQ) {
+                  bool withQ, bool withRows) {
   const StreamShape S = stream_shape(p->nx, p->ny, p->nz);
   const long long L = (long long)p->nx * p->ny * p->nz, Lp = S.Lp;
   const int nM = p->nM, nS = p->nSensors;
@@ -1274,6 +1237,8 @@ void stream_carve(const std::function<void *(size_t)> &take, mcb_heat_state *s, 
   s->uniY = S.ny <= kColMaxN ? (uint8_t *)take((size_t)S.px * S.nz * col_warps(S.ny)) : nullptr;
   s->uniZ = S.nz <= kColMaxN ? (uint8_t *)take((size_t)S.px * S.ny * col_warps(S.nz)) : nullptr;
   (void)nS;
+  s->rowX = nullptr;
+  if (withRows && rows_supported(S.nx, S.ny, S.nz)) rows_carve(take, s);
 }
 
 // Uploads M (pitched), the neighbourhood code, T (pitched deviations from the mean input
@@ -1323,6 +1288,7 @@ struct StreamStepper {
   int K = 8, XG = 16, gX = 1, gY = 1, gZ = 1;
   size_t xs = 0;
   bool colY = true, colZ = true;
+  const mcb_heat_state *rows = nullptr;  // step with the coded-row passes (heat_rows.cu)
 };
 
 // Per-call set-up of the streamed stepper on a state: the per-call tables (H = dt/2 c in FP32, as
@@ -1364,10 +1330,18 @@ mcb_status stream_setup(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *
   h.nS = nS; h.sIdx = s->sIdx; h.sW = s->sW; h.sens = sens; h.stepCounter = s->step; h.err = s->step + 1;
   s->lastW = h.W;
 
+  k.S = S;
+  if (s->rowX) {
+    bool coded = false;
+    MCB_TRY(rows_build(ctx, s, p, &coded));
+    if (coded) {
+      k.rows = s;
+      return MCB_OK;
+    }
+  }
   h.uniX = s->uniX;
   h.uniY = s->uniY;
   h.uniZ = s->uniZ;
-  k.S = S;
   k.maps = s->maps;
   k.K = x_chunk(S.nx);
   k.XG = x_lanes(S.nx);
@@ -1400,6 +1374,10 @@ mcb_status stream_setup(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *
 
 // Enqueues one DG-ADI step (X, Y and Z passes).
 void stream_step_launch(const StreamStepper &k, cudaStream_t q) {
+  if (k.rows) {
+    rows_step_launch(k.rows, k.h, q);
+    return;
+  }
   const StreamMaps &mp = *k.maps;
   const StreamDev &h = k.h;
   const StreamShape &S = k.S;
