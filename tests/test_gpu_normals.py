@@ -53,3 +53,18 @@ def test_device_normals_match_host(shape, d, ls, tol):
     edge = _interface(M1, n)
     ang = np.arccos(np.clip(np.sum(_unit(host)[:, edge] * _unit(dev)[:, edge], axis=0), -1, 1))
     assert np.max(ang) <= tol, np.max(ang)
+
+
+@pytest.mark.parametrize("shape", [(9, 300, 5), (130, 7, 12), (5, 4, 900), (3, 64, 65), (257, 2, 8)])
+def test_line_transforms_at_edges(shape):
+    """Smoothed normals where the tiles of the line transforms end: axes that are no multiple of the 8
+    outputs per thread, axes of several rounds (over 128 outputs), the 32-line tile (over 768), and a
+    last tile of few lines. The bound is that of the smoothed cases above."""
+    from mcmatlab_b200 import native
+    M1, n = _grid(shape, 2)
+    d = (0.0025, 0.002, 0.003)
+    host = prep.interface_normals(M1, n, *d, smoothingLengthScale=0.01)
+    dev = native.interface_normals(M1, n, *d, smoothingLengthScale=0.01)
+    edge = _interface(M1, n)
+    ang = np.arccos(np.clip(np.sum(_unit(host)[:, edge] * _unit(dev)[:, edge], axis=0), -1, 1))
+    assert np.max(ang) <= 1e-3, np.max(ang)
