@@ -12,6 +12,7 @@
 //   k1 = the first k < m0 with d'[k] > d0 (if any); start = k1 if it exists, else m0;
 //   m = the first index of the maximum of d' over [start, n); the next centre is m when
 //   d'[m] > d'[0], else point 0; m is carried to the next centre.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -20,6 +21,8 @@
 #include <vector>
 
 #include "internal.h"
+
+namespace cg = cooperative_groups;
 
 namespace mcb {
 namespace {
@@ -160,6 +163,162 @@ __global__ void ds_first_center_kernel(DsArgs a) {
   s.k1 = kNoIndex;
 }
 
+// The whole selection in one cooperative launch, for finite inputs of up to kOneMax points per SM
+// thread: every thread keeps P points (normalised coordinates, distance, bin) in registers, and one
+// grid barrier per centre replaces three launches that each read the points again. 300 000 points
+// into 40 bins: 0.20 ms on the device against 0.73 ms (18 us per centre, most of it the latency of the
+// three dependent launches).
+//
+// One pass serves the carried-index rule: besides the maximum over [m0, n) it takes the maximum over
+// all points and whether some k < m0 exceeds d0. If one does, every point before the first such k1 is
+// at most d0 < d'[k1], so the first index of the maximum over [k1, n) is that of the maximum over all
+// points. (NaN distances would break this; the host sends non-finite inputs to the kernels above.)
+struct DsRound {
+  unsigned long long all, high;  // keys of the maximum over all points and over k >= m0
+  unsigned int above;            // some k < m0 exceeds d0
+  float dZero;                   // distance of point 0
+};
+
+constexpr int kOneThreads = 1024, kOneMax = 8;
+
+template <int P>
+__global__ void __launch_bounds__(kOneThreads, 1) ds_one_kernel(DsArgs a, DsRound *rounds, int nBins) {
+  cg::grid_group grid = cg::this_grid();
+  __shared__ unsigned long long sAll, sHigh;
+  __shared__ unsigned int sAbove;
+  const long long k0 = blockIdx.x * (long long)kOneThreads + threadIdx.x, step = (long long)gridDim.x * kOneThreads;
+  float nv[P][3], d[P];
+  int bin[P];
+  // normalised coordinates of point k (rows that do not vary stay 0 and add nothing to a distance)
+  auto point = [&](long long k, float (&v)[3]) {
+#pragma unroll
+    for (int c = 0; c < 3; c++) v[c] = a.vary[c] ? __fmul_rn(a.par[3 * k + c], a.inv[c]) : 0.f;
+  };
+  // round r: this thread's maxima into rounds[r % 3]; the slot of round r + 2 is cleared behind the barrier
+  auto exchange = [&](int r, unsigned long long all, unsigned long long high, bool above) -> DsRound {
+    if (threadIdx.x == 0) {
+      sAll = sHigh = 0ull;
+      sAbove = 0u;
+    }
+    __syncthreads();
+    for (int o = 16; o > 0; o >>= 1) {
+      all = max(all, __shfl_down_sync(0xffffffffu, all, o));
+      high = max(high, __shfl_down_sync(0xffffffffu, high, o));
+    }
+    const bool any = __any_sync(0xffffffffu, above);
+    if ((threadIdx.x & 31) == 0) {
+      atomicMax(&sAll, all);
+      atomicMax(&sHigh, high);
+      if (any) sAbove = 1u;
+    }
+    __syncthreads();
+    DsRound *R = rounds + r % 3;
+    if (threadIdx.x == 0) {
+      atomicMax(&R->all, sAll);
+      atomicMax(&R->high, sHigh);
+      if (sAbove) atomicOr(&R->above, 1u);
+      if (blockIdx.x == 0) R->dZero = d[0];
+    }
+    grid.sync();
+    DsRound o;
+    o.all = __ldcg(&R->all);
+    o.high = __ldcg(&R->high);
+    o.above = __ldcg(&R->above);
+    o.dZero = __ldcg(&R->dZero);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      DsRound *N = rounds + (r + 2) % 3;
+      N->all = N->high = 0ull;
+      N->above = 0u;
+    }
+    return o;
+  };
+  auto index_of = [](unsigned long long key) { return (long long)(0xFFFFFFFFull - (key & 0xFFFFFFFFull)); };
+  auto distance = [&](const float (&v)[3], const float (&c)[3]) {
+    float acc = 0.f;
+#pragma unroll
+    for (int q = 0; q < 3; q++)
+      if (a.vary[q]) acc = add_sq(acc, v[q] - c[q]);
+    return acc;
+  };
+  auto write_center = [&](int j, const float (&c)[3]) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      int r = 0;
+      for (int q = 0; q < 3; q++)
+        if (a.vary[q]) a.centers[3 * j + r++] = c[q];
+    }
+  };
+  // the first centre is the point farthest from the mean
+  unsigned long long best = 0ull;
+#pragma unroll
+  for (int i = 0; i < P; i++) {
+    const long long k = k0 + i * step;
+    d[i] = 0.f;
+    bin[i] = 1;
+    if (k < a.n) {
+      point(k, nv[i]);
+      best = max(best, dist_key(distance(nv[i], a.meanTerm), k));
+    }
+  }
+  DsRound R = exchange(0, best, 0ull, false);
+  float c[3];
+  point(index_of(R.all), c);
+  write_center(0, c);
+  best = 0ull;
+#pragma unroll
+  for (int i = 0; i < P; i++) {
+    const long long k = k0 + i * step;
+    if (k < a.n) {
+      d[i] = distance(nv[i], c);
+      best = max(best, dist_key(d[i], k));
+    }
+  }
+  if (nBins > 1) {
+    R = exchange(1, best, 0ull, false);
+    long long next = index_of(R.all), m0 = 0;
+    float d0 = R.dZero;
+    for (int j = 1; j < nBins; j++) {
+      point(next, c);
+      write_center(j, c);
+      unsigned long long all = 0ull, high = 0ull;
+      bool above = false;
+#pragma unroll
+      for (int i = 0; i < P; i++) {
+        const long long k = k0 + i * step;
+        if (k < a.n) {
+          const float acc = distance(nv[i], c);
+          if (acc < d[i]) {
+            d[i] = acc;
+            bin[i] = j + 1;
+          }
+          const unsigned long long key = dist_key(d[i], k);
+          all = max(all, key);
+          if (k >= m0) high = max(high, key);
+          else above |= d[i] > d0;
+        }
+      }
+      if (j + 1 == nBins) break;  // the last centre needs no successor
+      R = exchange(j + 1, all, high, above);
+      const unsigned long long key = R.above ? R.all : R.high;
+      m0 = index_of(key);
+      d0 = __uint_as_float((unsigned int)(key >> 32));
+      next = d0 > R.dZero ? m0 : 0;
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < P; i++) {
+    const long long k = k0 + i * step;
+    if (k < a.n) a.bin[k] = (uint8_t)bin[i];
+  }
+}
+
+template <int P>
+mcb_status ds_one_launch(mcb_ctx *ctx, DsArgs a, DsRound *rounds, int nBins) {
+  const int blocks = (int)((a.n + (long long)kOneThreads * P - 1) / ((long long)kOneThreads * P));
+  void *args[] = {&a, &rounds, &nBins};
+  MCB_CUDA(ctx, cudaLaunchCooperativeKernel((const void *)ds_one_kernel<P>, dim3(blocks), dim3(kOneThreads), args, 0, ctx->stream));
+  return MCB_OK;
+}
+
 }  // namespace
 }  // namespace mcb
 
@@ -196,7 +355,7 @@ extern "C" mcb_status mcb_downsample_params(mcb_ctx *ctx, const float *paramVals
   cudaStream_t st = ctx->stream;
   auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
   const size_t bytes = al(12 * (size_t)n) + 3 * al(4 * (size_t)n) + al(4 * (size_t)n) + al((size_t)n) +
-                       al(12 * (size_t)nBins) + al(sizeof(DsState));
+                       al(12 * (size_t)nBins) + al(sizeof(DsState)) + al(3 * sizeof(DsRound));
   void *block = nullptr;
   MCB_TRY(pool_get(ctx, SLOT_DOWNSAMPLE, bytes, &block));
   char *cur = (char *)block;
@@ -217,7 +376,24 @@ extern "C" mcb_status mcb_downsample_params(mcb_ctx *ctx, const float *paramVals
   s0.k1 = kNoIndex;
   MCB_CUDA(ctx, cudaMemcpyAsync(a.s, &s0, sizeof(DsState), cudaMemcpyHostToDevice, st));
   const int grid = (int)std::max<long long>(1, std::min<long long>((n + 255) / 256, (long long)ctx->num_sms * 8));
-  if (a.rows > 0) {
+  // finite normalised coordinates and few enough points: the one-launch selection (a block per SM is
+  // always co-resident). Points fill half the SMs first, then registers: 300 000 points take 202 us with 4
+  // points per thread on 74 SMs, 251 us with 2 on 147 (a round is mostly its barrier and the blocks'
+  // atomics) and 236 us with 8 on 37.
+  bool one = a.rows > 0 && n <= (long long)ctx->num_sms * kOneThreads * kOneMax;
+  for (int c = 0; c < 3; c++)
+    one = one && std::isfinite(sm[c]) && std::isfinite(a.meanTerm[c]) &&
+          std::isfinite(std::max(std::fabs(mx[c]), std::fabs(mn[c])) * (a.vary[c] ? a.inv[c] : 1.0f));
+  if (one) {
+    DsRound *rounds = (DsRound *)take(3 * sizeof(DsRound));
+    MCB_CUDA(ctx, cudaMemsetAsync(rounds, 0, 3 * sizeof(DsRound), st));
+    const long long half = (long long)((ctx->num_sms + 1) / 2) * kOneThreads, per = (n + half - 1) / half;
+    if (per <= 1) MCB_TRY(ds_one_launch<1>(ctx, a, rounds, nBins));
+    else if (per <= 2) MCB_TRY(ds_one_launch<2>(ctx, a, rounds, nBins));
+    else if (per <= 4) MCB_TRY(ds_one_launch<4>(ctx, a, rounds, nBins));
+    else MCB_TRY(ds_one_launch<8>(ctx, a, rounds, nBins));
+    MCB_CUDA(ctx, cudaGetLastError());
+  } else if (a.rows > 0) {
     ds_init_kernel<<<grid, 256, 0, st>>>(a);
     ds_first_center_kernel<<<1, 1, 0, st>>>(a);
     ds_first_kernel<<<grid, 256, 0, st>>>(a);
