@@ -46,6 +46,7 @@ struct KernelArgs {
   // none is alive), so the divergent launch code runs once for a group of lanes.
   int refillMin;   // free lanes a warp waits for before launching new packets
   int scatterMin;  // waiting lanes before roulette + scattering run
+  int lanes;       // lanes of a warp that take packets (fewer where the packets do not fill the grid)
 };
 
 __device__ __forceinline__ unsigned long long global_ns() {
@@ -95,13 +96,17 @@ __device__ __forceinline__ unsigned long long fetch_packet(const KernelArgs &a) 
 }
 
 
-// Launch bounds: the plain kernel runs 4 blocks of 256 per SM at 64 registers (about 100 bytes
-// of spill stores; measured 3-9% more packets/s than 3 blocks at 80 registers without spills);
+// Variants (F): the packet state that only deposition criteria or times of flight read (event
+// counters, replay state, the time) is compiled out where no instance asks for it, which takes
+// the plain kernel from 56 bytes of spills to none at its 64 registers and shortens the loop's code
+// (100^3 cube, 1e6 packets: 6.3 -> 5.2 ms together with the scattering rule below).
+// Launch bounds: the plain kernel runs 4 blocks of 256 per SM at 64 registers (3 blocks at 80 registers
+// 5.6 ms, 5 at 48 with spills 6.0 ms, 4 blocks 5.2 ms);
 // the gradient variant runs 3 blocks without spills (at 64 registers it ran slower). The gradient
 // variant keeps its per-packet state (path length L_m and scattering count k_m per medium) and
 // its per-thread box partial sums in dynamic shared memory, one column per thread
 // (grad_smem_bytes), so that it holds 3 blocks per SM; the medium index selects the row directly.
-template <bool GRAD>
+template <bool GRAD, int F>
 __global__ void __launch_bounds__(256, GRAD ? 3 : 4) transport_kernel(KernelArgs a) {
   // single-instance runs read the instance and its medium table from shared memory
   __shared__ Inst sInst;
@@ -154,11 +159,11 @@ __global__ void __launch_bounds__(256, GRAD ? 3 : 4) transport_kernel(KernelArgs
   }
   Photon P;
   P.alive = false;
-  P.inbox = false;
+  P.inbox = P.turned = false;
   const Inst *I = single ? &sInst : a.insts;
   bool replay = false;
   bool started = false;
-  bool retired = false;
+  bool retired = (int)(threadIdx.x & 31) >= a.lanes;
   float wfinal = 0.f;
   float acc = 0.f;  // deposit run in one voxel (a few sub-steps)
   int accj = -1;
@@ -183,7 +188,7 @@ __global__ void __launch_bounds__(256, GRAD ? 3 : 4) transport_kernel(KernelArgs
         }
         boxC = 0.f;
       }
-      if (I->eol && !replay && I->NFR && criteria_met(P, *I)) {
+      if ((F & kFeatCrit) && I->eol && !replay && I->NFR && criteria_met<F>(P, *I)) {
         replay = true;
         wfinal = P.weight;
         relaunch = true;
@@ -217,7 +222,7 @@ __global__ void __launch_bounds__(256, GRAD ? 3 : 4) transport_kernel(KernelArgs
       P.pidlo = (uint32_t)pid;
       P.pidhi = (uint32_t)(pid >> 32);
       P.draw = 0;
-      const bool ok = launch_packet(P, *I);
+      const bool ok = launch_packet<true>(P, *I);
       if (ok || relaunch) voxel_props(P, *I);
       if (fresh) {
         if (ok) {
@@ -244,7 +249,12 @@ __global__ void __launch_bounds__(256, GRAD ? 3 : 4) transport_kernel(KernelArgs
       if (P.stepLeft > 0) {
         const int mj = GRAD ? P.med : 0;
         const float wpre = GRAD ? P.weight : 0.f;
-        const float s = propagate(P, *I);
+        if (P.turned) {
+          direction_changed(P, *I);
+          P.turned = false;
+        }
+        // (a cyclic wrap moves the packet after it turned, so variants with cyclic boundaries form D at once)
+        const float s = propagate<!(F & kFeatTime)>(P, *I);
         steps++;
         const float absorb = P.weight * one_minus_exp_neg(P.mua * s);
         P.weight -= absorb;
@@ -274,7 +284,7 @@ __global__ void __launch_bounds__(256, GRAD ? 3 : 4) transport_kernel(KernelArgs
           if (replay) {
             c = wfinal * absorb;
             dep = true;
-          } else if (!I->eol && criteria_met(P, *I)) {
+          } else if (!(F & kFeatCrit) || (!I->eol && criteria_met<F>(P, *I))) {
             c = absorb;
             dep = true;
           }
@@ -289,7 +299,7 @@ __global__ void __launch_bounds__(256, GRAD ? 3 : 4) transport_kernel(KernelArgs
           }
         }
         if (!P.sameVoxel) {
-          const bool tele = check_escape(P, *I, !replay);
+          const bool tele = check_escape<F>(P, *I, !replay);
           if (GRAD && !P.alive && P.kec != 0 && P.i[2] < 0 && nGR > 0) {
             // reflectance: escaping weight W on the top face, d/dmua_m = -L_m W,
             // d/dmus_m = (k_m / mus_m - L_m) W
@@ -324,13 +334,14 @@ __global__ void __launch_bounds__(256, GRAD ? 3 : 4) transport_kernel(KernelArgs
     //    until enough lanes of its warp are waiting too, or no lane can take a sub-step, so the
     //    long scattering code runs with most lanes active. A packet's events and random draws do
     //    not change, only when its warp performs them. The group size (a.scatterMin) is a launch
-    //    parameter of the autotuner; against single-lane scattering, groups of 8 gave the plain
-    //    kernel 9.5% more packets/s on the 100^3 cube.
+    //    parameter of the autotuner, but at most a quarter of the lanes still alive: in a thinned-out
+    //    warp (few packets, the end of a run) waiting for a full group only adds latency (half of the
+    //    lanes: 322 us on a 30^3 grid of 1e4 packets, a quarter 292, an eighth 289 but 5% more on full warps).
     {
       const bool want = P.alive && !(P.stepLeft > 0);
       const unsigned waiting = __ballot_sync(0xffffffffu, want);
       const unsigned stepping = __ballot_sync(0xffffffffu, P.alive && P.stepLeft > 0);
-      if (want && (__popc(waiting) >= a.scatterMin || stepping == 0)) {
+      if (want && (__popc(waiting) >= min(a.scatterMin, (__popc(waiting | stepping) + 3) >> 2) || stepping == 0)) {
         if (P.weight < kThreshold) {
           if (rnd(P, *I) <= kChance) P.weight /= kChance;
           else P.alive = false;
@@ -340,7 +351,7 @@ __global__ void __launch_bounds__(256, GRAD ? 3 : 4) transport_kernel(KernelArgs
             sGK[P.med * bd + tid] += 1.f;
             if (boxC > 0.f) sGE[P.med * bd + tid] += boxC;
           }
-          scatter(P, *I);
+          scatter<true>(P, *I);
         }
       }
     }
@@ -389,6 +400,8 @@ __global__ void scale_kernel(const double *acc, double inv, float *out, long lon
 // Example paths (MCmatlablib.c:465-514, updatePaths calls in launchPhoton/propagatePhoton/
 // scatterPhoton/checkEscape): packets 0, 1, 2, ... of the first instance are replayed serially
 // by one thread and their vertices recorded, NaN-separated, until nPaths paths are finished.
+constexpr int kFeatAll = kFeatCrit | kFeatTime;
+
 struct PathWriter {
   double *data;
   long long cap, n;
@@ -414,7 +427,7 @@ __device__ void path_add(PathWriter &W, const Photon &P, const Inst &I, int nanC
 
 __device__ void path_update(PathWriter &W, const Photon &P, const Inst &I, bool teleported) {
   if (W.n > W.cap) return;
-  if (I.eol || criteria_met(P, I)) path_add(W, P, I, W.started ? (teleported ? 1 : 0) : 2);
+  if (I.eol || criteria_met<kFeatAll>(P, I)) path_add(W, P, I, W.started ? (teleported ? 1 : 0) : 2);
 }
 
 __global__ void example_paths_kernel(const Inst *inst, int nPaths, unsigned long long maxPackets, double *data,
@@ -430,18 +443,18 @@ __global__ void example_paths_kernel(const Inst *inst, int nPaths, unsigned long
     P.pidhi = (uint32_t)(pid >> 32);
     P.draw = 0;
     W.started = false;
-    if (!launch_packet(P, I)) continue;
+    if (!launch_packet<false>(P, I)) continue;
     path_update(W, P, I, false);
     voxel_props(P, I);
     while (P.alive) {
       while (P.alive && P.stepLeft > 0) {
-        const float s = propagate(P, I);
+        const float s = propagate<false>(P, I);
         const float absorb = P.weight * one_minus_exp_neg(P.mua * s);
         P.weight -= absorb;
         path_update(W, P, I, false);
         if (!P.sameVoxel) {
-          const bool tele = check_escape(P, I, false);
-          if (tele && (I.eol || criteria_met(P, I))) path_update(W, P, I, true);
+          const bool tele = check_escape<kFeatAll>(P, I, false);
+          if (tele && (I.eol || criteria_met<kFeatAll>(P, I))) path_update(W, P, I, true);
           if (P.alive) voxel_props_crossed(P, I, tele);
         }
         if (++P.nsteps >= kMaxFreeSteps) P.alive = false;
@@ -451,12 +464,12 @@ __global__ void example_paths_kernel(const Inst *inst, int nPaths, unsigned long
         else P.alive = false;
       }
       if (P.alive) {
-        scatter(P, I);
+        scatter<false>(P, I);
         path_update(W, P, I, false);
       }
     }
     if (W.started) {
-      if (I.eol && !criteria_met(P, I)) W.n = startN;  // deletePhotonPath
+      if (I.eol && !criteria_met<kFeatAll>(P, I)) W.n = startN;  // deletePhotonPath
       else finished++;
     }
   }
@@ -908,14 +921,14 @@ int size_class(long long voxels, bool grad, bool batched) {
   return c + (grad ? 16 : 0) + (batched ? 32 : 0);
 }
 
-// The autotuner's override, else the class's tuned parameters, else the autotuner's choices on the
-// 100^3 cube (refill 16, scatter 8: 6.83 ms for 1e6 packets against 7.14 ms at 8, 8) and on the
-// 256^3 gradient cube (12, 12).
+// The autotuner's override, else the class's tuned parameters, else the defaults: (12, 8) on the
+// 100^3 cube (5.07 ms for 1e6 packets, 5.16 at 16, 8) and (12, 12) for gradients; all pairs from (8, 8)
+// to (16, 12) lie within 2% of each other.
 mcb_mc_launch launch_params(const mcb_ctx *ctx, int cls, bool grad) {
   if (ctx->force.refillMin > 0) return ctx->force;
   const auto it = ctx->tuned.find(cls);
   if (it != ctx->tuned.end()) return it->second;
-  return grad ? mcb_mc_launch{12, 12} : mcb_mc_launch{16, 8};
+  return grad ? mcb_mc_launch{12, 12} : mcb_mc_launch{12, 8};
 }
 
 mcb_status launch_transport(mcb_ctx *ctx, Arena &ar, const std::vector<Inst> &insts, bool openEnded,
@@ -954,12 +967,26 @@ mcb_status launch_transport(mcb_ctx *ctx, Arena &ar, const std::vector<Inst> &in
     a.scatterMin = L.scatterMin;
   }
   const size_t dynSmem = grad ? grad_smem_bytes(insts[0].nM, insts[0].nR, 256) : 0;
-  if (grad)
-    MCB_CUDA(ctx, cudaFuncSetAttribute(transport_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dynSmem));
+  // the variant with what any of the instances asks for
+  int feat = 0;
+  for (const Inst &I : insts) {
+    if (I.crit) feat |= kFeatAll;
+    if (I.bt == 3 || (I.image && I.LCres1 > 1)) feat |= kFeatTime;
+  }
+  void (*kernel)(KernelArgs) = grad ? (feat ? transport_kernel<true, kFeatTime> : transport_kernel<true, 0>)
+                               : feat & kFeatCrit ? transport_kernel<false, kFeatAll>
+                               : feat             ? transport_kernel<false, kFeatTime>
+                                                  : transport_kernel<false, 0>;
+  if (grad) MCB_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dynSmem));
   int blocksPerSm = 0;
-  MCB_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocksPerSm, grad ? transport_kernel<true> : transport_kernel<false>, 256, dynSmem));
+  MCB_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocksPerSm, kernel, 256, dynSmem));
   if (blocksPerSm < 1) blocksPerSm = 1;
   const int grid = ctx->num_sms * blocksPerSm;
+  // fewer packets than lanes: spread over all warps, a few lanes of each. Such a run lasts as long as its
+  // longest packet, and a sub-step of a warp with 3 packets takes less time than one with 32 (30^3 grid, 1e4
+  // packets: 479 us packed into 313 warps, 295 us spread over 4736).
+  a.lanes = 32;
+  if (!openEnded) a.lanes = (int)std::max<unsigned long long>(1, std::min<unsigned long long>(32, (a.totalPackets + grid * 8 - 1) / (grid * 8)));
   if (ar.overflow) return set_error(ctx, MCB_ENOMEM, "internal: device arena too small");
   if (openEnded && seconds > 0) {
     // the deadline is taken on the device clock (%globaltimer, ns) right before the launch
@@ -971,8 +998,7 @@ mcb_status launch_transport(mcb_ctx *ctx, Arena &ar, const std::vector<Inst> &in
     a.deadlineNs = now + (unsigned long long)(seconds * 1e9);
   }
   MCB_CUDA(ctx, cudaEventRecord(ctx->ev0, st));
-  if (grad) transport_kernel<true><<<grid, 256, dynSmem, st>>>(a);
-  else transport_kernel<false><<<grid, 256, 0, st>>>(a);
+  kernel<<<grid, 256, dynSmem, st>>>(a);
   MCB_CUDA(ctx, cudaGetLastError());
   MCB_CUDA(ctx, cudaEventRecord(ctx->ev1, st));
   unsigned long long tail[3];
