@@ -70,8 +70,10 @@ extern "C" mcb_status mcb_ctx_create(int device, mcb_ctx **out) {
   }
   int *h = nullptr;
   if (cudaHostAlloc((void **)&h, sizeof(int) * 4, cudaHostAllocMapped) != cudaSuccess ||
-      cudaHostGetDevicePointer((void **)&ctx->cancel_dev, h, 0) != cudaSuccess) {
+      cudaHostGetDevicePointer((void **)&ctx->cancel_dev, h, 0) != cudaSuccess ||
+      cudaHostAlloc(&ctx->pin, mcb::kPinBytes, cudaHostAllocDefault) != cudaSuccess) {
     cudaGetLastError();
+    if (h) cudaFreeHost(h);
     cudaStreamDestroy(ctx->stream);
     delete ctx;
     return MCB_ECUDA;
@@ -90,6 +92,7 @@ extern "C" mcb_status mcb_ctx_destroy(mcb_ctx *ctx) {
     if (b.ptr) cudaFree(b.ptr);
   if (ctx->heat) mcb_heat_state_destroy(ctx->heat);
   if (ctx->cancel_host) cudaFreeHost((void *)ctx->cancel_host);
+  if (ctx->pin) cudaFreeHost(ctx->pin);
   if (ctx->ev0) cudaEventDestroy(ctx->ev0);
   if (ctx->ev1) cudaEventDestroy(ctx->ev1);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);

@@ -433,8 +433,8 @@ mcb_status check_params(mcb_ctx *ctx, const mcb_heat_params *p) {
   for (int m = 0; m < p->nM; m++)
     if (!(p->A[m] >= 0) || !(p->E[m] >= 0)) return set_error(ctx, MCB_EINVAL, "A and E must be non-negative");
   // every kernel indexes the media tables with M: reject indices beyond them
-  for (long long k = 0; k < L; k++)
-    if (p->M[k] >= p->nM) return set_error(ctx, MCB_EINVAL, "M holds a medium index outside 0..nM-1 (voxel %lld)", k);
+  const long long k = first_outside(p->M, L, 0, p->nM - 1);
+  if (k >= 0) return set_error(ctx, MCB_EINVAL, "M holds a medium index outside 0..nM-1 (voxel %lld)", k);
   if (std::min(yz_tile_width((int)ny), yz_tile_width((int)nz)) == 0)
     return set_error(ctx, MCB_EINVAL, "y or z lines longer than the shared-memory tile limit");
   if (x_lines((int)nx) == 0) return set_error(ctx, MCB_EINVAL, "x lines longer than the shared-memory limit");
@@ -554,13 +554,12 @@ mcb_status state_alloc(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *p
 void damage_table(const mcb_heat_params *p, double base, float2 *out) { heat_damage_table(p, base, out); }
 
 // Uploads the media/coefficients/source of p and the state T, Omega (host pointers).
-mcb_status state_upload(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *p, const float *T, const float *Omega) {
+mcb_status state_upload(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *p, const float *T, const float *Omega,
+                        double base) {
   cudaStream_t st = ctx->stream;
   const long long L = s->L;
   const int nM = s->nM;
-  double sum = 0.0;
-  for (long long k = 0; k < L; k++) sum += T[k];
-  s->base = sum / (double)L;
+  s->base = base;
   std::vector<double> logA(nM);
   for (int m = 0; m < nM; m++) logA[m] = std::log(p->A[m]);
   std::vector<float2> dmg(nM);
@@ -662,10 +661,10 @@ void heat_damage_table(const mcb_heat_params *p, double base, float2 *out) {
 mcb_status heat_check_params(mcb_ctx *ctx, const mcb_heat_params *p) { return check_params(ctx, p); }
 
 mcb_status heat_state_init(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *p, const float *T,
-                           const float *Omega) {
+                           const float *Omega, double base) {
   const bool damage = Omega != nullptr;
   if (!state_fits(s, p, damage, false)) MCB_TRY(state_alloc(ctx, s, p, damage));
-  return state_upload(ctx, s, p, T, Omega);
+  return state_upload(ctx, s, p, T, Omega, base);
 }
 
 void heat_state_release(mcb_heat_state *s) { free_state_buffers(s); }
@@ -728,14 +727,14 @@ extern "C" mcb_status mcb_heat_forward(mcb_ctx *ctx, const mcb_heat_params *p, f
   }
   if (stream_supported(p->nx, p->ny, p->nz)) {
     if (!state_fits(s, p, damage, true)) MCB_TRY(stream_alloc(ctx, s, p, damage));
-    MCB_TRY(stream_upload(ctx, s, p, T, Omega));
+    MCB_TRY(stream_upload(ctx, s, p, T, Omega, heat_mean(T, (long long)p->nx * p->ny * p->nz)));
     if (p->lightsOn) MCB_TRY(stream_upload_q(ctx, s, p->dTdt_abs));
     MCB_TRY(sensor_buffers(ctx, s, p));
     MCB_TRY(stream_step(ctx, s, p, s->sens, sensorTemps, maxMediaTemps, true));
     return stream_download(ctx, s, T, Omega);
   }
   if (!state_fits(s, p, damage, false)) MCB_TRY(state_alloc(ctx, s, p, damage));
-  MCB_TRY(state_upload(ctx, s, p, T, Omega));
+  MCB_TRY(state_upload(ctx, s, p, T, Omega, heat_mean(T, s->L)));
   MCB_TRY(state_step(ctx, s, p, sensorTemps, maxMediaTemps));
   return state_download(ctx, s, T, Omega);
 }
@@ -752,11 +751,11 @@ extern "C" mcb_status mcb_heat_state_create(mcb_ctx *ctx, const mcb_heat_params 
   mcb_status st;
   if (stream_supported(p->nx, p->ny, p->nz)) {
     st = stream_alloc(ctx, s, p, Omega != nullptr);
-    if (st == MCB_OK) st = stream_upload(ctx, s, p, T, Omega);
+    if (st == MCB_OK) st = stream_upload(ctx, s, p, T, Omega, heat_mean(T, (long long)p->nx * p->ny * p->nz));
     if (st == MCB_OK && p->lightsOn) st = stream_upload_q(ctx, s, p->dTdt_abs);
   } else {
     st = state_alloc(ctx, s, p, Omega != nullptr);
-    if (st == MCB_OK) st = state_upload(ctx, s, p, T, Omega);
+    if (st == MCB_OK) st = state_upload(ctx, s, p, T, Omega, heat_mean(T, s->L));
   }
   if (st != MCB_OK) {
     free_state_buffers(s);
@@ -951,7 +950,7 @@ extern "C" mcb_status mcb_heat_forward_static(mcb_ctx *ctx, const mcb_heat_param
     s.ctx = ctx;
     s.streamed = true;
     mcb_status rc = stream_maps(ctx, &s);
-    if (rc == MCB_OK) rc = stream_upload(ctx, &s, p, T, Omega);
+    if (rc == MCB_OK) rc = stream_upload(ctx, &s, p, T, Omega, heat_mean(T, (long long)p->nx * p->ny * p->nz));
     if (rc == MCB_OK && p->lightsOn) rc = stream_upload_q(ctx, &s, p->dTdt_abs);
     if (rc == MCB_OK && p->nSensors) {
       const cudaError_t e1 = cudaMemcpyAsync(s.sIdx, p->tempSensorCornerIdxs, 8 * (size_t)p->nSensors,
@@ -981,9 +980,7 @@ extern "C" mcb_status mcb_heat_forward_static(mcb_ctx *ctx, const mcb_heat_param
   const long long L = s.L, nt = p->steps;
   const int nM = s.nM, nS = p->nSensors;
   // upload (the same steps as the allocating path; logA is staged on the stack: nM <= 256)
-  double sum = 0.0;
-  for (long long k = 0; k < L; k++) sum += T[k];
-  s.base = sum / (double)L;
+  s.base = heat_mean(T, L);
   double logA[256];
   for (int m = 0; m < nM; m++) logA[m] = std::log(p->A[m]);
   float2 dmg[256];
@@ -1028,13 +1025,13 @@ extern "C" mcb_status mcb_heat_forward_static(mcb_ctx *ctx, const mcb_heat_param
 }
 
 namespace mcb {
-mcb_status stream_state_create(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *p, const float *T) {
+mcb_status stream_state_create(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *p, const float *T, double base) {
   s->ctx = ctx;
   // The TMA-staged passes, not the coded rows: the adjoint's peak terms take each voxel's hottest
   // step, and where a voxel's temperature barely moves the last bits of T decide which step that
   // is. (With the coded rows the gradients of a 120 x 111 x 90 run moved by 0.6% through such ties.)
   MCB_TRY(stream_alloc(ctx, s, p, false, false));
-  MCB_TRY(stream_upload(ctx, s, p, T, nullptr));
+  MCB_TRY(stream_upload(ctx, s, p, T, nullptr, base));
   if (p->lightsOn) MCB_TRY(stream_upload_q(ctx, s, p->dTdt_abs));
   return MCB_OK;
 }

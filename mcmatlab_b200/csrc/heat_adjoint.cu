@@ -28,6 +28,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <vector>
 
 #include "heat_host.h"
@@ -742,11 +743,23 @@ void weight_list(const float *w, long long L, std::vector<int> &idx, std::vector
   idx.clear();
   val.clear();
   if (!w) return;
-  for (long long v = 0; v < L; v++)
-    if (w[v] != 0.f) {
-      idx.push_back((int)v);
-      val.push_back(w[v]);
+  // blocks of zeros are skipped by the or of their bits (the host compiler vectorises it)
+  constexpr int B = 64;
+  for (long long b = 0; b < L; b += B) {
+    const long long e = std::min(b + B, L);
+    uint32_t any = 0;
+    for (long long v = b; v < e; v++) {
+      uint32_t u;
+      std::memcpy(&u, w + v, 4);
+      any |= u << 1;  // without the sign: -0 is a zero
     }
+    if (!any) continue;
+    for (long long v = b; v < e; v++)
+      if (w[v] != 0.f) {
+        idx.push_back((int)v);
+        val.push_back(w[v]);
+      }
+  }
 }
 
 }  // namespace
@@ -780,7 +793,11 @@ extern "C" mcb_status mcb_heat_adjoint(mcb_ctx *ctx, const mcb_heat_params *pin,
   cudaStream_t st = ctx->stream;
   mcb_heat_state s;
   s.ctx = ctx;
-  mcb_status rc = heat_state_init(ctx, &s, &p, T0, nullptr);
+  // one running sum, as the derivative of a peak depends on T's last bits where a voxel's maxima tie
+  double sum = 0.0;
+  for (long long k = 0; k < L; k++) sum += T0[k];
+  const double base = sum / (double)L;
+  mcb_status rc = heat_state_init(ctx, &s, &p, T0, nullptr, base);
   if (rc != MCB_OK) {
     heat_state_release(&s);
     return rc;
@@ -892,7 +909,7 @@ extern "C" mcb_status mcb_heat_adjoint(mcb_ctx *ctx, const mcb_heat_params *pin,
   // sweep keeps the factored state's LU pivots for its transposed solves.
   int *pIdxS = pIdxD;
   if (stream_supported(p.nx, p.ny, p.nz)) {
-    rc = stream_state_create(ctx, &ss, &p, T0);
+    rc = stream_state_create(ctx, &ss, &p, T0, base);
     if (rc == MCB_OK) rc = stream_stepper_new(ctx, &ss, &p, &sk);
     if (rc != MCB_OK) {
       if (sk) stream_stepper_free(sk);
@@ -902,11 +919,8 @@ extern "C" mcb_status mcb_heat_adjoint(mcb_ctx *ctx, const mcb_heat_params *pin,
     }
     if (nP) {
       // the peak list's voxels in the streamed state's pitched grid
-      std::vector<int> pIdxP(nP);
-      for (int k = 0; k < nP; k++) pIdxP[k] = (int)stream_pitched_index(&ss, pIdx[k]);
       pIdxS = (int *)take(4 * (size_t)nP);
-      ADJ_CUDA(cudaMemcpyAsync(pIdxS, pIdxP.data(), 4 * (size_t)nP, cudaMemcpyHostToDevice, st));
-      ADJ_CUDA(cudaStreamSynchronize(st));
+      stream_pitched_indices(&ss, pIdxD, pIdxS, nP, st);
     }
   }
   // forward sweep: checkpoints every K steps, running maxima of the peak list

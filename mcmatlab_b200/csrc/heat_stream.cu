@@ -973,6 +973,10 @@ __global__ void merge_omega_p_kernel(float *Omega, const float *dOmega, Pitch P,
     Omega[v] = (float)((double)Omega[v] + (double)dOmega[P.p(v)]);
 }
 
+__global__ void pitched_index_kernel(const int *dense, int *pitched, int n, Pitch P) {
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) pitched[k] = (int)P.p(dense[k]);
+}
+
 __global__ void final_sensors_p_kernel(StreamDev h) { record_sensors_p(h, *h.stepCounter); }
 
 // H <- hdt * c in place (FP32 products, as the stepper forms its coefficients), the diagonal table
@@ -1241,17 +1245,16 @@ void stream_carve(const std::function<void *(size_t)> &take, mcb_heat_state *s, 
   if (withRows && rows_supported(S.nx, S.ny, S.nz)) rows_carve(take, s);
 }
 
-// Uploads M (pitched), the neighbourhood code, T (pitched deviations from the mean input
+// Uploads M (pitched), the neighbourhood code, T (pitched deviations from `base`, the mean input
 // temperature) and Omega; clears the padding of every pitched grid.
-mcb_status stream_upload(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *p, const float *T, const float *Omega) {
+mcb_status stream_upload(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *p, const float *T, const float *Omega,
+                         double base) {
   cudaStream_t st = ctx->stream;
   const StreamShape &S = s->shape;
   const long long L = (long long)S.nx * S.ny * S.nz;
   const Pitch P{S.nx, S.ny, S.nz, S.px};
   const int grid = ctx->num_sms * 8;
-  double sum = 0.0;
-  for (long long k = 0; k < L; k++) sum += T[k];
-  s->base = sum / (double)L;
+  s->base = base;
   MCB_CUDA(ctx, cudaMemsetAsync(s->T, 0, 4 * S.Lp, st));
   MCB_CUDA(ctx, cudaMemsetAsync(s->A, 0, 4 * S.Lp, st));
   if (s->Q) MCB_CUDA(ctx, cudaMemsetAsync(s->Q, 0, 4 * S.Lp, st));
@@ -1416,11 +1419,9 @@ void stream_dense_set(mcb_ctx *ctx, mcb_heat_state *s, const float *dense, cudaS
   to_pitched_dev_kernel<<<ctx->num_sms * 8, 256, 0, st>>>(dense, s->T, 0.0, Pitch{S.nx, S.ny, S.nz, S.px});
 }
 
-long long stream_pitched_index(const mcb_heat_state *s, long long v) {
+void stream_pitched_indices(const mcb_heat_state *s, const int *dense, int *pitched, int n, cudaStream_t st) {
   const StreamShape &S = s->shape;
-  const long long nxy = (long long)S.nx * S.ny;
-  const long long iz = v / nxy, r = v - iz * nxy, iy = r / S.nx, ix = r - iy * S.nx;
-  return ix + (iy + iz * S.ny) * S.px;
+  pitched_index_kernel<<<std::max(1, std::min(1184, (n + 255) / 256)), 256, 0, st>>>(dense, pitched, n, Pitch{S.nx, S.ny, S.nz, S.px});
 }
 
 // Runs p->steps steps on the device-resident streamed state. Sensor and maximum outputs go to

@@ -29,6 +29,7 @@ struct mcb_ctx {
   std::vector<DevBuf> pool;             // indexed slots, grow-only
   int num_sms = 0;
   mcb_heat_state *heat = nullptr;  // state reused by mcb_heat_forward
+  void *pin = nullptr;             // kPinBytes of page-locked host memory: small results leave through it
   double lastKernelMs = 0.0;        // device time of the last stepping / transport loop
   // transport launch parameters: tuned per size class (mcb_mc_autotune, or read from the tuning
   // file at context creation), and an override used while the autotuner calibrates
@@ -43,6 +44,28 @@ mcb_status set_error(mcb_ctx *ctx, mcb_status st, const char *fmt, ...);
 
 // Returns a device buffer for `slot` of at least `bytes` (contents undefined).
 mcb_status pool_get(mcb_ctx *ctx, int slot, size_t bytes, void **out);
+
+constexpr size_t kPinBytes = (size_t)1 << 20;
+
+// Index of the first of p[0..n) outside lo..hi, or -1. Whole blocks are judged by one maximum, which
+// the host compiler vectorises; only a block that holds such a value is searched. (A loop that
+// returns at the first one takes 0.7 ns per voxel: 0.8 ms of a 5 ms transport call on 100^3 voxels.)
+inline long long first_outside(const uint8_t *p, long long n, int lo, int hi) {
+  if (hi < lo) return n > 0 ? 0 : -1;
+  const uint8_t base = (uint8_t)lo, span = (uint8_t)(hi - lo);
+  for (long long b = 0; b < n; b += 16384) {
+    const long long e = b + 16384 < n ? b + 16384 : n;
+    uint8_t most = 0;
+    for (long long k = b; k < e; k++) {
+      const uint8_t d = (uint8_t)(p[k] - base);
+      most = d > most ? d : most;
+    }
+    if (most > span)
+      for (long long k = b; k < e; k++)
+        if (p[k] < lo || p[k] > hi) return k;
+  }
+  return -1;
+}
 
 // Reads the transport launch parameters tuned for this GPU from the file MCB_TUNE_FILE names.
 void tune_file_load(mcb_ctx *ctx);

@@ -392,9 +392,23 @@ __global__ void normalize_nfr_kernel(const double *acc, const uint8_t *M0, const
     out[k] = (float)(acc[k] / (scale * (double)med[M0[k]].x));
 }
 
-__global__ void scale_kernel(const double *acc, double inv, float *out, long long n) {
-  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x)
-    out[k] = (float)(acc[k] * inv);
+// The remaining tallies of one wavelength, scaled and written as float: pieces one after the other.
+struct ScalePiece {
+  const double *acc;
+  double inv;
+  long long n;
+};
+struct ScalePieces {
+  ScalePiece p[8];
+  int count;
+};
+__global__ void scale_kernel(ScalePieces s, float *out) {
+  for (int q = 0; q < s.count; q++) {
+    const ScalePiece p = s.p[q];
+    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < p.n; k += (long long)gridDim.x * blockDim.x)
+      out[k] = (float)(p.acc[k] * p.inv);
+    out += p.n;
+  }
 }
 
 // Example paths (MCmatlablib.c:465-514, updatePaths calls in launchPhoton/propagatePhoton/
@@ -629,12 +643,16 @@ mcb_status validate(mcb_ctx *ctx, const mcb_mc_model *m) {
   }
   if (m->sourceDistribution) {
     const long long LL = (long long)m->nx * m->ny * m->nz * m->nL;
-    for (long long k = 0; k < LL; k++)
-      if (!(m->sourceDistribution[k] >= 0) || !std::isfinite(m->sourceDistribution[k]))
-        return set_error(ctx, MCB_EINVAL, "sourceDistribution must be finite and non-negative");
+    // non-negative and finite by its bits (the sign of zero aside): one or per value, vectorised
+    uint32_t bad = 0;
+    for (long long k = 0; k < LL; k++) {
+      uint32_t u;
+      std::memcpy(&u, m->sourceDistribution + k, 4);
+      bad |= (uint32_t)(u > 0x7F7FFFFFu) & (uint32_t)(u != 0x80000000u);
+    }
+    if (bad) return set_error(ctx, MCB_EINVAL, "sourceDistribution must be finite and non-negative");
   }
-  for (long long k = 0; k < L; k++)
-    if (m->M[k] < 1 || m->M[k] > m->nM) return set_error(ctx, MCB_EINVAL, "M holds a medium index outside 1..nM");
+  if (first_outside(m->M, L, 1, std::min(m->nM, 255)) >= 0) return set_error(ctx, MCB_EINVAL, "M holds a medium index outside 1..nM");
   if (mismatched && !m->interfaceNormals)
     return set_error(ctx, MCB_EINVAL, "refractive indices differ between media but interfaceNormals is NULL");
   if (m->useLightCollector && m->LC_res < 1 && std::isfinite(m->LC_f))
@@ -735,15 +753,8 @@ mcb_status build_plan(mcb_ctx *ctx, Arena &ar, ModelPlan &pl, uint32_t stream) {
       med[q] = make_float4((float)m->mua[q], (float)m->mus[q], (float)m->g[q], (float)m->n[q]);
       cdx[q] = std::isnan(m->CDFidx[q]) ? 0 : (int)(unsigned char)m->CDFidx[q];
     }
-  pl.med = ar.take<float4>(med.size());
-  pl.cdfidx = ar.take<int>(cdx.size());
-  pl.CDFs = ar.take<float>(std::max<int64_t>(m->nCDFelems, 1));
-  if (ar.overflow) return set_error(ctx, MCB_ENOMEM, "internal: device arena too small");
-  MCB_CUDA(ctx, cudaMemcpyAsync(pl.med, med.data(), med.size() * sizeof(float4), cudaMemcpyHostToDevice, st));
-  MCB_CUDA(ctx, cudaMemcpyAsync(pl.cdfidx, cdx.data(), cdx.size() * sizeof(int), cudaMemcpyHostToDevice, st));
   std::vector<float> cdfs(std::max<int64_t>(m->nCDFelems, 1), 0.f);
   for (int64_t k = 0; k < m->nCDFelems; k++) cdfs[k] = (float)m->CDFs[k];
-  MCB_CUDA(ctx, cudaMemcpyAsync(pl.CDFs, cdfs.data(), cdfs.size() * 4, cudaMemcpyHostToDevice, st));
   // beam
   std::vector<float> FP1{0.f}, FP2{0.f}, AI1{0.f}, AI2{0.f};
   if (!pl.useS && m->sourceType >= 4) {
@@ -759,10 +770,24 @@ mcb_status build_plan(mcb_ctx *ctx, Arena &ar, ModelPlan &pl, uint32_t stream) {
   beam.insert(beam.end(), FP2.begin(), FP2.end());
   beam.insert(beam.end(), AI1.begin(), AI1.end());
   beam.insert(beam.end(), AI2.begin(), AI2.end());
-  pl.beam = ar.take<float>(beam.size());
+  // the small tables in one copy: media, phase-function indices and CDFs, beam
+  {
+    const size_t nMed = med.size() * sizeof(float4), nIdx = cdx.size() * 4, nCdf = cdfs.size() * 4, nBeam = beam.size() * 4;
+    std::vector<char> all(nMed + nIdx + nCdf + nBeam);
+    std::memcpy(all.data(), med.data(), nMed);
+    std::memcpy(all.data() + nMed, cdx.data(), nIdx);
+    std::memcpy(all.data() + nMed + nIdx, cdfs.data(), nCdf);
+    std::memcpy(all.data() + nMed + nIdx + nCdf, beam.data(), nBeam);
+    char *d = ar.take<char>(all.size());
+    if (ar.overflow) return set_error(ctx, MCB_ENOMEM, "internal: device arena too small");
+    pl.med = (float4 *)d;
+    pl.cdfidx = (int *)(d + nMed);
+    pl.CDFs = (float *)(d + nMed + nIdx);
+    pl.beam = (float *)(d + nMed + nIdx + nCdf);
+    MCB_CUDA(ctx, cudaMemcpyAsync(d, all.data(), all.size(), cudaMemcpyHostToDevice, st));
+  }
   if (pl.useS) pl.S = ar.take<double>((size_t)(L + 1) * nL);
   if (ar.overflow) return set_error(ctx, MCB_ENOMEM, "internal: device arena too small");
-  MCB_CUDA(ctx, cudaMemcpyAsync(pl.beam, beam.data(), beam.size() * 4, cudaMemcpyHostToDevice, st));
   // distributed source CDFs (MCmatlab.c:626-629), per wavelength, in double
   pl.power.assign(nL, 0.0);
   if (pl.useS) {
@@ -789,17 +814,14 @@ mcb_status build_plan(mcb_ctx *ctx, Arena &ar, ModelPlan &pl, uint32_t stream) {
   pl.Lz = nx * ny;
   pl.Lzn = m->boundaryType == 2 ? nx * ny * kKillRange * kKillRange : nx * ny;
   pl.niPer = 2 * pl.Lx + 2 * pl.Ly + pl.Lz + pl.Lzn;
+  const size_t zero0 = (ar.used + 255) & ~(size_t)255;  // the accumulators follow one another: one memset
   if (m->calcNFR) pl.accNFR = ar.take<double>((size_t)L * nL);
   if (pl.Lim) pl.accImg = ar.take<double>((size_t)pl.Lim * nL);
   if (pl.Lff) pl.accFF = ar.take<double>((size_t)pl.Lff * nL);
   pl.accNI = ar.take<double>((size_t)pl.niPer * nL);
   pl.ctr = ar.take<unsigned long long>(kCtr * (size_t)nL);
   if (ar.overflow) return set_error(ctx, MCB_ENOMEM, "internal: device arena too small");
-  if (pl.accNFR) MCB_CUDA(ctx, cudaMemsetAsync(pl.accNFR, 0, 8 * (size_t)L * nL, st));
-  if (pl.accImg) MCB_CUDA(ctx, cudaMemsetAsync(pl.accImg, 0, 8 * (size_t)pl.Lim * nL, st));
-  if (pl.accFF) MCB_CUDA(ctx, cudaMemsetAsync(pl.accFF, 0, 8 * (size_t)pl.Lff * nL, st));
-  MCB_CUDA(ctx, cudaMemsetAsync(pl.accNI, 0, 8 * (size_t)pl.niPer * nL, st));
-  MCB_CUDA(ctx, cudaMemsetAsync(pl.ctr, 0, 8 * kCtr * (size_t)nL, st));
+  MCB_CUDA(ctx, cudaMemsetAsync(ar.base + zero0, 0, ar.used - zero0, st));
 
   // beam basis (MCmatlab.c:579-589)
   const double tb = pl.useS ? 0 : m->theta, pb = pl.useS ? 0 : m->phi, psib = pl.useS ? 0 : m->psi;
@@ -940,13 +962,17 @@ mcb_status launch_transport(mcb_ctx *ctx, Arena &ar, const std::vector<Inst> &in
   for (int k = 0; k < n; k++) first[k + 1] = first[k] + insts[k].count;
   std::vector<Inst> host = insts;
   for (int k = 0; k < n; k++) host[k].first = first[k];
-  Inst *dInst = ar.take<Inst>(n);
-  unsigned long long *dFirst = ar.take<unsigned long long>(n + 1);
-  unsigned long long *scratch = ar.take<unsigned long long>(4);  // [0] next packet, [1] steps, [2] status, [3] clock
+  // one copy: [n] instances, [n + 1] first packets, scratch: [0] next packet, [1] steps, [2] status, [3] clock
+  static_assert(sizeof(Inst) % 8 == 0, "the packet ranges follow the instances");
+  const size_t nInst = sizeof(Inst) * n, nFirst = 8 * ((size_t)n + 1);
+  std::vector<char> all(nInst + nFirst + 32, 0);
+  std::memcpy(all.data(), host.data(), nInst);
+  std::memcpy(all.data() + nInst, first.data(), nFirst);
+  char *d = ar.take<char>(all.size());
   if (ar.overflow) return set_error(ctx, MCB_ENOMEM, "internal: device arena too small");
-  MCB_CUDA(ctx, cudaMemcpyAsync(dInst, host.data(), sizeof(Inst) * n, cudaMemcpyHostToDevice, st));
-  MCB_CUDA(ctx, cudaMemcpyAsync(dFirst, first.data(), 8 * (n + 1), cudaMemcpyHostToDevice, st));
-  MCB_CUDA(ctx, cudaMemsetAsync(scratch, 0, 32, st));
+  Inst *dInst = (Inst *)d;
+  unsigned long long *dFirst = (unsigned long long *)(d + nInst), *scratch = dFirst + n + 1;
+  MCB_CUDA(ctx, cudaMemcpyAsync(d, all.data(), all.size(), cudaMemcpyHostToDevice, st));
   KernelArgs a;
   a.insts = dInst;
   a.instFirst = dFirst;
@@ -1001,7 +1027,7 @@ mcb_status launch_transport(mcb_ctx *ctx, Arena &ar, const std::vector<Inst> &in
   kernel<<<grid, 256, dynSmem, st>>>(a);
   MCB_CUDA(ctx, cudaGetLastError());
   MCB_CUDA(ctx, cudaEventRecord(ctx->ev1, st));
-  unsigned long long tail[3];
+  unsigned long long *tail = (unsigned long long *)ctx->pin;
   MCB_CUDA(ctx, cudaMemcpyAsync(tail, scratch, 24, cudaMemcpyDeviceToHost, st));
   MCB_CUDA(ctx, cudaStreamSynchronize(st));
   float ms = 0.f;
@@ -1021,7 +1047,8 @@ mcb_status finish_plan(mcb_ctx *ctx, Arena &ar, ModelPlan &pl, double *nPhCum, d
   const int grid = ctx->num_sms * 8;
   std::vector<unsigned long long> ctr(kCtr * (size_t)nL);
   r->freeStepCuts = r->freeStepCutWeight = 0.0;
-  MCB_CUDA(ctx, cudaMemcpyAsync(ctr.data(), pl.ctr, 8 * ctr.size(), cudaMemcpyDeviceToHost, st));
+  const bool ctrPinned = 8 * ctr.size() <= kPinBytes;
+  MCB_CUDA(ctx, cudaMemcpyAsync(ctrPinned ? ctx->pin : ctr.data(), pl.ctr, 8 * ctr.size(), cudaMemcpyDeviceToHost, st));
   if (r->tallies) {
     // the FP64 tallies as accumulated (the normalisation below reads them, it does not change them)
     const TallyLayout t = tally_layout(m);
@@ -1031,6 +1058,7 @@ mcb_status finish_plan(mcb_ctx *ctx, Arena &ar, ModelPlan &pl, double *nPhCum, d
     MCB_CUDA(ctx, cudaMemcpyAsync(r->tallies + t.ni, pl.accNI, 8 * (size_t)pl.niPer * nL, cudaMemcpyDeviceToHost, st));
   }
   MCB_CUDA(ctx, cudaStreamSynchronize(st));
+  if (ctrPinned) std::memcpy(ctr.data(), ctx->pin, 8 * ctr.size());
   if (r->tallies) {
     const TallyLayout t = tally_layout(m);
     for (int iL = 0; iL < nL; iL++) {
@@ -1039,7 +1067,9 @@ mcb_status finish_plan(mcb_ctx *ctx, Arena &ar, ModelPlan &pl, double *nPhCum, d
     }
   }
   const double V = m->dx * m->dy * m->dz;
-  float *stage = ar.take<float>(std::max<long long>(std::max<long long>(L, pl.Lim), std::max<long long>(pl.Lff, pl.niPer)));
+  float *stage = pl.accNFR ? ar.take<float>(L) : nullptr;
+  const long long small = pl.Lff + pl.Lim + pl.niPer;
+  float *stage2 = ar.take<float>(small);
   if (ar.overflow) return set_error(ctx, MCB_ENOMEM, "internal: device arena too small");
   for (int iL = 0; iL < nL; iL++) {
     const double nPh = (double)ctr[kCtr * iL], nCol = (double)ctr[kCtr * iL + 1];
@@ -1054,44 +1084,58 @@ mcb_status finish_plan(mcb_ctx *ctx, Arena &ar, ModelPlan &pl, double *nPhCum, d
     if (pl.useS) nf /= pl.power[iL];
     else if (m->sourceType == 2 && (m->boundaryType == 0 || m->boundaryType == 2)) nf /= kKillRange * kKillRange;
     if (nPh == 0) nf = 1.0;  // nothing launched: tallies are zero
+    // far field, image and faces: scaled by one launch, and out through the page-locked buffer in one
+    // copy where they fit it
+    ScalePieces sp{};
+    float *dst[8];
+    auto piece = [&](const double *src, float *to, long long cnt, double inv) {
+      if (!to || cnt <= 0) return;
+      sp.p[sp.count] = ScalePiece{src, inv, cnt};
+      dst[sp.count++] = to + (size_t)iL * cnt;
+    };
+    if (pl.accFF) piece(pl.accFF + (size_t)iL * pl.Lff, r->farField, pl.Lff, 1.0 / nf);
+    if (pl.accImg) {
+      const long long Lp = (long long)m->LC_res * m->LC_res;
+      const double fs = std::isfinite(m->LC_f) ? m->LC_fieldSize : m->LC_NA;
+      piece(pl.accImg + (size_t)iL * pl.Lim, r->image, pl.Lim, Lp > 1 ? 1.0 / (fs * fs / Lp * nf) : 1.0 / nf);
+    }
+    const double *ni = pl.accNI + (size_t)iL * pl.niPer;
+    auto face = [&](const double *src, float *to, long long cnt, double area) { piece(src, to, cnt, 1.0 / (area * nf)); };
+    if (m->boundaryType == 1) {
+      face(ni, r->NI_xpos, pl.Lx, m->dy * m->dz);
+      face(ni + pl.Lx, r->NI_xneg, pl.Lx, m->dy * m->dz);
+      face(ni + 2 * pl.Lx, r->NI_ypos, pl.Ly, m->dx * m->dz);
+      face(ni + 2 * pl.Lx + pl.Ly, r->NI_yneg, pl.Ly, m->dx * m->dz);
+      face(ni + 2 * pl.Lx + 2 * pl.Ly, r->NI_zpos, pl.Lz, m->dx * m->dy);
+      face(ni + 2 * pl.Lx + 2 * pl.Ly + pl.Lz, r->NI_zneg, pl.Lz, m->dx * m->dy);
+    } else if (m->boundaryType == 2) {
+      face(ni, r->NI_zneg, pl.Lzn, m->dx * m->dy);
+    } else if (m->boundaryType == 3) {
+      face(ni, r->NI_zpos, pl.Lz, m->dx * m->dy);
+      face(ni + pl.Lz, r->NI_zneg, pl.Lz, m->dx * m->dy);
+    }
+    long long total = 0;
+    for (int q = 0; q < sp.count; q++) total += sp.p[q].n;
+    const bool pinned = 4 * (size_t)total <= kPinBytes;
+    if (total) {
+      scale_kernel<<<grid, 256, 0, st>>>(sp, stage2);
+      if (pinned) {
+        MCB_CUDA(ctx, cudaMemcpyAsync(ctx->pin, stage2, 4 * total, cudaMemcpyDeviceToHost, st));
+      } else {
+        long long o = 0;
+        for (int q = 0; q < sp.count; o += sp.p[q].n, q++)
+          MCB_CUDA(ctx, cudaMemcpyAsync(dst[q], stage2 + o, 4 * sp.p[q].n, cudaMemcpyDeviceToHost, st));
+      }
+    }
     if (pl.accNFR && r->NFR) {
       normalize_nfr_kernel<<<grid, 256, 0, st>>>(pl.accNFR + (size_t)iL * L, pl.M0, pl.med + (size_t)iL * m->nM, V * nf, stage, L);
       MCB_CUDA(ctx, cudaMemcpyAsync(r->NFR + (size_t)iL * L, stage, 4 * L, cudaMemcpyDeviceToHost, st));
-      MCB_CUDA(ctx, cudaStreamSynchronize(st));
     }
-    if (pl.accFF && r->farField) {
-      scale_kernel<<<grid, 256, 0, st>>>(pl.accFF + (size_t)iL * pl.Lff, 1.0 / nf, stage, pl.Lff);
-      MCB_CUDA(ctx, cudaMemcpyAsync(r->farField + (size_t)iL * pl.Lff, stage, 4 * pl.Lff, cudaMemcpyDeviceToHost, st));
-      MCB_CUDA(ctx, cudaStreamSynchronize(st));
-    }
-    if (pl.accImg && r->image) {
-      const long long Lp = (long long)m->LC_res * m->LC_res;
-      const double fs = std::isfinite(m->LC_f) ? m->LC_fieldSize : m->LC_NA;
-      const double inv = Lp > 1 ? 1.0 / (fs * fs / Lp * nf) : 1.0 / nf;
-      scale_kernel<<<grid, 256, 0, st>>>(pl.accImg + (size_t)iL * pl.Lim, inv, stage, pl.Lim);
-      MCB_CUDA(ctx, cudaMemcpyAsync(r->image + (size_t)iL * pl.Lim, stage, 4 * pl.Lim, cudaMemcpyDeviceToHost, st));
-      MCB_CUDA(ctx, cudaStreamSynchronize(st));
-    }
-    const double *ni = pl.accNI + (size_t)iL * pl.niPer;
-    auto face = [&](const double *src, float *dst, long long cnt, double area) -> mcb_status {
-      if (!dst) return MCB_OK;
-      scale_kernel<<<grid, 256, 0, st>>>(src, 1.0 / (area * nf), stage, cnt);
-      MCB_CUDA(ctx, cudaMemcpyAsync(dst + (size_t)iL * cnt, stage, 4 * cnt, cudaMemcpyDeviceToHost, st));
-      MCB_CUDA(ctx, cudaStreamSynchronize(st));
-      return MCB_OK;
-    };
-    if (m->boundaryType == 1) {
-      MCB_TRY(face(ni, r->NI_xpos, pl.Lx, m->dy * m->dz));
-      MCB_TRY(face(ni + pl.Lx, r->NI_xneg, pl.Lx, m->dy * m->dz));
-      MCB_TRY(face(ni + 2 * pl.Lx, r->NI_ypos, pl.Ly, m->dx * m->dz));
-      MCB_TRY(face(ni + 2 * pl.Lx + pl.Ly, r->NI_yneg, pl.Ly, m->dx * m->dz));
-      MCB_TRY(face(ni + 2 * pl.Lx + 2 * pl.Ly, r->NI_zpos, pl.Lz, m->dx * m->dy));
-      MCB_TRY(face(ni + 2 * pl.Lx + 2 * pl.Ly + pl.Lz, r->NI_zneg, pl.Lz, m->dx * m->dy));
-    } else if (m->boundaryType == 2) {
-      MCB_TRY(face(ni, r->NI_zneg, pl.Lzn, m->dx * m->dy));
-    } else if (m->boundaryType == 3) {
-      MCB_TRY(face(ni, r->NI_zpos, pl.Lz, m->dx * m->dy));
-      MCB_TRY(face(ni + pl.Lz, r->NI_zneg, pl.Lz, m->dx * m->dy));
+    MCB_CUDA(ctx, cudaGetLastError());
+    MCB_CUDA(ctx, cudaStreamSynchronize(st));
+    if (total && pinned) {
+      const float *o = (const float *)ctx->pin;
+      for (int q = 0; q < sp.count; o += sp.p[q].n, q++) std::memcpy(dst[q], o, 4 * sp.p[q].n);
     }
   }
   return MCB_OK;

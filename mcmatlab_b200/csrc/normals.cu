@@ -268,8 +268,8 @@ extern "C" mcb_status mcb_interface_normals(mcb_ctx *ctx, int32_t nx, int32_t ny
   if (smooth && std::max(nx, std::max(ny, nz)) > kNrmMaxLine)
     return set_error(ctx, MCB_EINVAL, "smoothing supports axes of at most %d voxels", kNrmMaxLine);
   const long long L = (long long)nx * ny * nz;
-  for (long long v = 0; v < L; v++)
-    if (M1[v] < 1 || M1[v] > nM) return set_error(ctx, MCB_EINVAL, "M1[%lld] = %d is not a medium in 1..%d", v, (int)M1[v], nM);
+  const long long v = first_outside(M1, L, 1, nM <= 255 ? nM : 255);
+  if (v >= 0) return set_error(ctx, MCB_EINVAL, "M1[%lld] = %d is not a medium in 1..%d", v, (int)M1[v], nM);
   MCB_CUDA(ctx, cudaSetDevice(ctx->device));
   cudaStream_t st = ctx->stream;
   const size_t fbytes = 4 * (size_t)L;
