@@ -447,7 +447,7 @@ mcb_status check_params(mcb_ctx *ctx, const mcb_heat_params *p) {
 namespace {
 
 void free_state_buffers(mcb_heat_state *s) {
-  if (s->block) cudaFree(s->block);
+  if (s->block && s->slot < 0) cudaFree(s->block);
   if (s->sens) cudaFree(s->sens);
   if (s->sIdx) cudaFree(s->sIdx);
   delete s->maps;
@@ -459,13 +459,20 @@ void free_state_buffers(mcb_heat_state *s) {
   s->streamed = false;
 }
 
+// The state's one allocation: its own, or its slot of the context's pool.
+mcb_status state_block(mcb_ctx *ctx, mcb_heat_state *s, size_t need) {
+  if (s->slot >= 0) return pool_get(ctx, s->slot, need, &s->block);
+  MCB_CUDA(ctx, cudaMalloc(&s->block, need));
+  return MCB_OK;
+}
+
 // Streamed state (heat_stream.cu) for p's grid in one allocation, with its TMA descriptors.
 mcb_status stream_alloc(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *p, bool damage, bool rows = true) {
   free_state_buffers(s);
   size_t need = 0;
   mcb_heat_state probe{};
   stream_carve([&](size_t b) { need += (b + 255) & ~(size_t)255; return (void *)nullptr; }, &probe, p, damage, true, rows);
-  MCB_CUDA(ctx, cudaMalloc(&s->block, need));
+  MCB_TRY(state_block(ctx, s, need));
   char *cur = (char *)s->block;
   stream_carve([&](size_t b) { char *q = cur; cur += (b + 255) & ~(size_t)255; return (void *)q; }, s, p, damage, true, rows);
   s->streamed = true;
@@ -517,7 +524,7 @@ mcb_status state_alloc(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *p
                       24 * L /*fb*/ + L /*nb*/ + 4 * L /*Sz*/ + (damage ? 8 * L : 0) + L + 12 * (size_t)nM * nM +
                       24 * (size_t)nM /*logA E dmg*/ + 4 * (size_t)nM + 64 + 25 * 256;
   free_state_buffers(s);
-  MCB_CUDA(ctx, cudaMalloc(&s->block, need));
+  MCB_TRY(state_block(ctx, s, need));
   char *cur = (char *)s->block;
   auto take = [&](size_t bytes) {
     char *q = cur;

@@ -24,6 +24,8 @@
 // K - 1 inner states of a segment recomputed during the reverse sweep (K = ceil(steps /
 // nCheckpoints); a segment's end states are checkpoints), and six grid-sized work arrays. With
 // nCheckpoints = steps every state is stored and nothing is recomputed.
+#include <cooperative_groups.h>
+#include <cooperative_groups/reduce.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -32,6 +34,8 @@
 #include <vector>
 
 #include "heat_host.h"
+
+namespace cg = cooperative_groups;
 
 namespace mcb {
 namespace {
@@ -58,6 +62,7 @@ struct AdjDev {
   const float *pW;
   const int *pStep;  // step (1..steps) at which each peak-list voxel reached its maximum
   int step;          // n + 1 of the step being reversed
+  int zChunk;        // planes per block of the assembly
 };
 
 // Objective terms at T^{n+1}: damage (weight w, increment dt A exp(-E / R Tmid)) contributes
@@ -220,7 +225,6 @@ constexpr int kZHN = kZHX * kZHY;  // halo tile (340)
 constexpr int kZCN = kZX * kZY;    // centre tile, one thread per column (256)
 constexpr int kZA1 = kZY * kZHX;   // x-halo tile (272)
 constexpr int kZR2 = kZHY * kZX;   // y-halo tile (320)
-constexpr int kZChunk = 25;        // planes per block
 static_assert(kZHN <= 2 * kZCN && kZR2 <= 2 * kZCN && kZA1 <= 2 * kZCN, "two staging slots per thread cover every tile");
 
 // out = U - dt/2 D_d (U - T^n) at one voxel along the line direction d, from its value u, T^n
@@ -241,6 +245,15 @@ __device__ __forceinline__ float recon_point(const float *C, int nM, float hdt, 
     if (hasr) dd += C[m + nM * mr] * ((ur - tr) - w);
   }
   return u - hdt * dd;
+}
+
+// Adds v to sums[k]: the lanes of a warp that meet here with the same k add up first. On an interface
+// plane all 256 columns of a block meet in one entry, and a shared-memory FP64 atomic is a
+// compare-and-swap loop.
+__device__ __forceinline__ void add_pair(double *sums, int k, float v) {
+  const auto group = cg::labeled_partition(cg::coalesced_threads(), k);
+  const double s = cg::reduce(group, (double)v, cg::plus<double>());
+  if (group.thread_rank() == 0) atomicAdd(&sums[k], s);
 }
 
 __global__ void __launch_bounds__(kZCN, 1024 / kZCN) adj_assemble_z_kernel(AdjDev a) {
@@ -321,8 +334,8 @@ __global__ void __launch_bounds__(kZCN, 1024 / kZCN) adj_assemble_z_kernel(AdjDe
       if (e < kZR2) sR2[slot][e] = pR2[q];
     }
   };
-  // this block's planes [z0, z1) (blockIdx.z: z chunks of kZChunk planes, for more blocks in flight)
-  const int z0 = blockIdx.z * kZChunk, z1 = min(nz, z0 + kZChunk);
+  // this block's planes [z0, z1) (blockIdx.z: z chunks, for more blocks in flight; adj_z_chunk)
+  const int z0 = blockIdx.z * a.zChunk, z1 = min(nz, z0 + a.zChunk);
   const float dt = h.dt, hdt = h.hdt;
   // A2 of plane p on the halo tile, into sA2[p & 1] (z neighbours from the ring)
   auto form_a2 = [&](int p) {
@@ -382,6 +395,8 @@ __global__ void __launch_bounds__(kZCN, 1024 / kZCN) adj_assemble_z_kernel(AdjDe
   const int ix = x0 + tx, iy = y0 + ty;
   const bool col = ix < nx && iy < ny;
   const int hc = (ty + 1) * kZHX + tx + 1;  // centre in the halo tile
+  // steps to the x and y neighbours (0: there is none)
+  const int xl = ix > 0 ? -1 : 0, xr = ix < nx - 1 ? 1 : 0, yl = iy > 0 ? -1 : 0, yr = iy < ny - 1 ? 1 : 0;
   // per plane, two phases: (1) assemble plane iz and form A2 of plane iz + 1; (2) form A1 of
   // plane iz + 1, stage the prefetched ring plane iz + 3 (into the slot of iz - 1) and r2 of plane
   // iz + 1, and start the loads of ring plane iz + 4 and r2 of plane iz + 2
@@ -403,39 +418,43 @@ __global__ void __launch_bounds__(kZCN, 1024 / kZCN) adj_assemble_z_kernel(AdjDe
         same[0] = same[1] = same[2] = 0.f;
       }
       float lam = r1v;
-      // all six neighbours present, of the voxel's medium, and none of them (nor the voxel)
-      // heat-sinked
-      const int lo = h.hs ? 2 : 1;
-      const bool interior = ix >= lo && ix < nx - lo && iy >= lo && iy < ny - lo && iz >= lo && iz < nz - lo &&
-                            sM[sc][hc - 1] == mv && sM[sc][hc + 1] == mv && sM[sc][hc - kZHX] == mv &&
-                            sM[sc][hc + kZHX] == mv && sM[sm][hc] == mv && sM[sp][hc] == mv;
-      if (interior) {
-        const float cx = cfs(mv, mv, 0), cy = cfs(mv, mv, 1), cz = cfs(mv, mv, 2);
-        const float r1xl = sR1[sc][hc - 1], r1xr = sR1[sc][hc + 1], r1yl = sR1[sc][hc - kZHX],
-                    r1yr = sR1[sc][hc + kZHX];
-        const float r1zl = sR1[sm][hc], r1zr = sR1[sp][hc];
-        const float r2yl = sR2[q1][ty * kZX + tx], r2yr = sR2[q1][(ty + 2) * kZX + tx];
-        const float r3zl = sR3[sm][t], r3zr = sR3[sp][t];
-        const float txl = sTN[sc][hc - 1], txr = sTN[sc][hc + 1], tyl = sTN[sc][hc - kZHX], tyr = sTN[sc][hc + kZHX];
-        const float tzl = sTN[sm][hc], tzr = sTN[sp][hc];
-        const float a1l = A1c[ty * kZHX + tx], a1r = A1c[ty * kZHX + tx + 2];
-        const float a2l = A2c[hc - kZHX], a2r = A2c[hc + kZHX];
-        const float tpl = sTP[sm][hc], tpr = sTP[sp][hc];
-        const float qy = dt * r1v - hdt * r2v, qz = dt * r1v - hdt * r3v;
-        lam += cx * hdt * (r1xl + r1xr - 2.f * r1v) +
-               cy * ((dt * r1yl - hdt * r2yl) + (dt * r1yr - hdt * r2yr) - 2.f * qy) +
-               cz * ((dt * r1zl - hdt * r3zl) + (dt * r1zr - hdt * r3zr) - 2.f * qz);
+      // Directions whose neighbours are of the voxel's own medium, no heat-sinked voxel about, take the
+      // difference form; a missing neighbour is the voxel itself, whose differences vanish. Only a direction
+      // across an interface takes the general form: the blocks of an interface plane, all whose columns
+      // do, decide how long the kernel runs.
+      const int zl = iz > 0 ? sm : sc, zr = iz < nz - 1 ? sp : sc;
+      const bool free = !h.hs || (ix >= 2 && ix < nx - 2 && iy >= 2 && iy < ny - 2 && iz >= 2 && iz < nz - 2);
+      const bool px = free && sM[sc][hc + xl] == mv && sM[sc][hc + xr] == mv;
+      const bool py = free && sM[sc][hc + yl * kZHX] == mv && sM[sc][hc + yr * kZHX] == mv;
+      const bool pz = free && sM[zl][hc] == mv && sM[zr][hc] == mv;
+      const float qy = dt * r1v - hdt * r2v, qz = dt * r1v - hdt * r3v;
+      if (px) {
+        const float r1xl = sR1[sc][hc + xl], r1xr = sR1[sc][hc + xr], txl = sTN[sc][hc + xl], txr = sTN[sc][hc + xr];
+        const float a1l = A1c[ty * kZHX + tx + 1 + xl], a1r = A1c[ty * kZHX + tx + 1 + xr];
+        lam += cfs(mv, mv, 0) * hdt * (r1xl + r1xr - 2.f * r1v);
         same[0] += hdt * r1v * ((txl + a1l) + (txr + a1r) - 2.f * (tv + a1v));
+      }
+      if (py) {
+        const float r1yl = sR1[sc][hc + yl * kZHX], r1yr = sR1[sc][hc + yr * kZHX];
+        const float r2yl = sR2[q1][(ty + 1 + yl) * kZX + tx], r2yr = sR2[q1][(ty + 1 + yr) * kZX + tx];
+        const float tyl = sTN[sc][hc + yl * kZHX], tyr = sTN[sc][hc + yr * kZHX];
+        const float a2l = A2c[hc + yl * kZHX], a2r = A2c[hc + yr * kZHX];
+        lam += cfs(mv, mv, 1) * ((dt * r1yl - hdt * r2yl) + (dt * r1yr - hdt * r2yr) - 2.f * qy);
         same[1] += dt * r1v * (tyl + tyr - 2.f * tv) + hdt * r2v * ((a2l - tyl) + (a2r - tyr) - 2.f * (a2v - tv));
+      }
+      if (pz) {
+        const float r1zl = sR1[zl][hc], r1zr = sR1[zr][hc], r3zl = sR3[zl][t], r3zr = sR3[zr][t];
+        const float tzl = sTN[zl][hc], tzr = sTN[zr][hc], tpl = sTP[zl][hc], tpr = sTP[zr][hc];
+        lam += cfs(mv, mv, 2) * ((dt * r1zl - hdt * r3zl) + (dt * r1zr - hdt * r3zr) - 2.f * qz);
         same[2] += dt * r1v * (tzl + tzr - 2.f * tv) + hdt * r3v * ((tpl - tzl) + (tpr - tzr) - 2.f * (tpv - tv));
-        a.lamOut[v] = lam;
-        if (a.dQ && !a.dQinX) a.dQ[v] += dt * r1v;
-      } else {
+      }
+      if (!(px && py && pz)) {
 #pragma unroll
         for (int d = 0; d < 3; d++) {
+          if (d == 0 ? px : (d == 1 ? py : pz)) continue;
           const int pos = d == 0 ? ix : (d == 1 ? iy : iz);
           const int n = d == 0 ? nx : (d == 1 ? ny : nz);
-          const float qv = d == 0 ? hdt * r1v : (d == 1 ? dt * r1v - hdt * r2v : dt * r1v - hdt * r3v);
+          const float qv = d == 0 ? hdt * r1v : (d == 1 ? qy : qz);
           const float pv = d == 0 ? tv + a1v : (d == 1 ? a2v - tv : tpv - tv);
 #pragma unroll
           for (int side = -1; side <= 1; side += 2) {
@@ -459,13 +478,13 @@ __global__ void __launch_bounds__(kZCN, 1024 / kZCN) adj_assemble_z_kernel(AdjDe
               else if (d == 1) contrib = dt * r1v * (tu - tv) + hdt * r2v * ((A2c[hu] - tu) - pv);
               else contrib = dt * r1v * (tu - tv) + hdt * r3v * ((sTP[rs][hc] - tu) - pv);
               if (mu == mv) same[d] += contrib;
-              else atomicAdd(&sdc[mv + mu * nM + d * nM2], (double)contrib);
+              else add_pair(sdc, mv + mu * nM + d * nM2, contrib);
             }
           }
         }
-        a.lamOut[v] = lam;
-        if (a.dQ && !a.dQinX && nsv) a.dQ[v] += dt * r1v;
       }
+      a.lamOut[v] = lam;
+      if (a.dQ && !a.dQinX && nsv) a.dQ[v] += dt * r1v;
     }
     __syncthreads();
     if (iz + 1 < z1) form_a1(iz + 1);
@@ -738,6 +757,17 @@ void adj_launch_yz(const AdjDev &a, bool zpass, int grid, cudaStream_t st) {
   else adj_solve_yz_kernel<TW, false><<<grid, 256, adj_yz_tile_bytes<TW>(a.h.ny) + 64, st>>>(a);
 }
 
+// Planes per block of the assembly, 25 on large grids (50 measured no faster): a block walks its chunk's
+// planes one after the other, four more being staged or formed before the first. Smaller grids take
+// shorter chunks, down to 5 planes, until the blocks make one and a half rounds of the `slots` that run
+// at a time: one round leaves the GPU to the blocks of interface planes, which take longest
+// (120 x 111 x 90 voxels: 129 us with 25 planes, 113 with 15, 91 with 9, 78 with 5).
+int adj_z_chunk(int tiles, int nz, int slots) {
+  int c = std::min(nz, 25);
+  while (c > 5 && (long long)tiles * ((nz + c - 1) / c) * 2 < 3ll * slots) c--;
+  return c;
+}
+
 // Compressed (index, weight) list of the nonzero entries of a per-voxel weight array.
 void weight_list(const float *w, long long L, std::vector<int> &idx, std::vector<float> &val) {
   idx.clear();
@@ -791,8 +821,11 @@ extern "C" mcb_status mcb_heat_adjoint(mcb_ctx *ctx, const mcb_heat_params *pin,
 
   MCB_CUDA(ctx, cudaSetDevice(ctx->device));
   cudaStream_t st = ctx->stream;
+  // both states live in the context's pool, as the work memory does: allocating and freeing them took
+  // 3 ms of each call on 1.2e6 voxels
   mcb_heat_state s;
   s.ctx = ctx;
+  s.slot = SLOT_ADJ_STATE;
   // one running sum, as the derivative of a peak depends on T's last bits where a voxel's maxima tie
   double sum = 0.0;
   for (long long k = 0; k < L; k++) sum += T0[k];
@@ -839,6 +872,7 @@ extern "C" mcb_status mcb_heat_adjoint(mcb_ctx *ctx, const mcb_heat_params *pin,
   float *pVal = (float *)take(4 * (size_t)std::max(nP, 1));
   int *pStepD = (int *)take(4 * (size_t)std::max(nP, 1));
   mcb_heat_state ss;  // streamed state of the forward sweeps (below)
+  ss.slot = SLOT_ADJ_STREAM;
   StreamStepper *sk = nullptr;
   auto fail = [&](mcb_status r) {
     if (sk) {
@@ -899,7 +933,9 @@ extern "C" mcb_status mcb_heat_adjoint(mcb_ctx *ctx, const mcb_heat_params *pin,
   if (rc == MCB_OK && nx <= 512) rc = adj_xline_setup(ctx, nx, &gridXL);
   if (rc != MCB_OK) return fail(rc);
   const int gridL = std::max(1, std::min(ctx->num_sms * 4, (std::max(nD, nP) + 255) / 256));
-  const dim3 gridZ((nx + kZX - 1) / kZX, (ny + kZY - 1) / kZY, (nz + kZChunk - 1) / kZChunk);
+  const int tilesZ = ((nx + kZX - 1) / kZX) * ((ny + kZY - 1) / kZY);
+  a.zChunk = adj_z_chunk(tilesZ, nz, ctx->num_sms * (1024 / kZCN));
+  const dim3 gridZ((nx + kZX - 1) / kZX, (ny + kZY - 1) / kZY, (nz + a.zChunk - 1) / a.zChunk);
   const size_t smemZ = (size_t)3 * nM * nM * (8 + 4);
   ADJ_CUDA(cudaFuncSetAttribute(adj_assemble_z_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemZ));
   a.dQinX = gridXL != 0;

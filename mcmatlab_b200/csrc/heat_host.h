@@ -66,6 +66,7 @@ struct mcb_heat_state {
   long long sensCap = 0;
   int sCap = 0;
   void *block = nullptr;
+  int slot = -1;  // >= 0: the block is this slot of the context's buffer pool, not the state's own
 };
 
 namespace mcb {

@@ -109,6 +109,8 @@ enum PoolSlot {
   SLOT_PROBE,
   SLOT_NORMALS,
   SLOT_DOWNSAMPLE,
+  SLOT_ADJ_STATE,   // the adjoint's factored and streamed states
+  SLOT_ADJ_STREAM,
   SLOT_BATCH_BASE = 40
 };
 
