@@ -456,7 +456,7 @@ void free_state_buffers(mcb_heat_state *s) {
   s->sens = s->sIdx = nullptr;
   s->sensCap = 0;
   s->sCap = 0;
-  s->streamed = false;
+  s->streamed = s->rowsOnly = false;
 }
 
 // The state's one allocation: its own, or its slot of the context's pool.
@@ -482,6 +482,8 @@ mcb_status stream_alloc(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *
   s->nM = p->nM;
   s->L = (long long)p->nx * p->ny * p->nz;
   s->damage = damage;
+  s->rowsOnly = !stream_supported(p->nx, p->ny, p->nz);
+  if (s->rowsOnly) return MCB_OK;  // no TMA-staged passes
   s->maps = new StreamMaps();
   return stream_maps(ctx, s);
 }
@@ -560,28 +562,55 @@ mcb_status state_alloc(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *p
 
 void damage_table(const mcb_heat_params *p, double base, float2 *out) { heat_damage_table(p, base, out); }
 
-// Uploads the media/coefficients/source of p and the state T, Omega (host pointers).
-mcb_status state_upload(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *p, const float *T, const float *Omega,
-                        double base) {
+// Uploads the media and coefficient tables of p (host pointers); waits for the copies.
+mcb_status state_upload_tables(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *p) {
   cudaStream_t st = ctx->stream;
-  const long long L = s->L;
   const int nM = s->nM;
-  s->base = base;
   std::vector<double> logA(nM);
   for (int m = 0; m < nM; m++) logA[m] = std::log(p->A[m]);
   std::vector<float2> dmg(nM);
   damage_table(p, s->base, dmg.data());
-  MCB_CUDA(ctx, cudaMemcpyAsync(s->stage, T, 4 * L, cudaMemcpyHostToDevice, st));
-  to_dev_kernel<<<ctx->num_sms * 8, 256, 0, st>>>(s->stage, s->T, s->base, L);
-  MCB_CUDA(ctx, cudaMemcpyAsync(s->M, p->M, L, cudaMemcpyHostToDevice, st));
-  if (p->dTdt_abs) MCB_CUDA(ctx, cudaMemcpyAsync(s->Q, p->dTdt_abs, 4 * L, cudaMemcpyHostToDevice, st));
-  if (s->Om && Omega) MCB_CUDA(ctx, cudaMemcpyAsync(s->Om, Omega, 4 * L, cudaMemcpyHostToDevice, st));
+  MCB_CUDA(ctx, cudaMemcpyAsync(s->M, p->M, s->L, cudaMemcpyHostToDevice, st));
   MCB_CUDA(ctx, cudaMemcpyAsync(s->c, p->dTdtperdeltaT, 12 * (size_t)nM * nM, cudaMemcpyHostToDevice, st));
   MCB_CUDA(ctx, cudaMemcpyAsync(s->logA, logA.data(), 8 * nM, cudaMemcpyHostToDevice, st));
   MCB_CUDA(ctx, cudaMemcpyAsync(s->E, p->E, 8 * nM, cudaMemcpyHostToDevice, st));
   MCB_CUDA(ctx, cudaMemcpyAsync(s->dmg, dmg.data(), 8 * nM, cudaMemcpyHostToDevice, st));
   MCB_CUDA(ctx, cudaStreamSynchronize(st));  // host buffers (logA, dmg) go out of scope
   s->factoredDt = -1.0;
+  return MCB_OK;
+}
+
+// Uploads the media/coefficients/source of p and the state T, Omega (host pointers).
+mcb_status state_upload(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *p, const float *T, const float *Omega,
+                        double base) {
+  cudaStream_t st = ctx->stream;
+  const long long L = s->L;
+  s->base = base;
+  MCB_CUDA(ctx, cudaMemcpyAsync(s->stage, T, 4 * L, cudaMemcpyHostToDevice, st));
+  to_dev_kernel<<<ctx->num_sms * 8, 256, 0, st>>>(s->stage, s->T, s->base, L);
+  if (p->dTdt_abs) MCB_CUDA(ctx, cudaMemcpyAsync(s->Q, p->dTdt_abs, 4 * L, cudaMemcpyHostToDevice, st));
+  if (s->Om && Omega) MCB_CUDA(ctx, cudaMemcpyAsync(s->Om, Omega, 4 * L, cudaMemcpyHostToDevice, st));
+  return state_upload_tables(ctx, s, p);
+}
+
+// A rowsOnly state whose row coefficients no longer fit the code tables (another dt or boundary type)
+// goes on as a factored one: T, the base and Omega stay on the device.
+mcb_status state_to_factored(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *p) {
+  mcb_heat_state f;
+  f.ctx = ctx;
+  MCB_TRY(state_alloc(ctx, &f, p, s->damage));
+  f.base = s->base;
+  stream_dense_copy(ctx, s, f.T, ctx->stream);
+  mcb_status rc = MCB_OK;
+  if (s->damage && cudaMemcpyAsync(f.Om, s->Om, 4 * s->L, cudaMemcpyDeviceToDevice, ctx->stream) != cudaSuccess)
+    rc = set_error(ctx, MCB_ECUDA, "copy of the damage state failed");
+  if (rc == MCB_OK) rc = state_upload_tables(ctx, &f, p);
+  if (rc != MCB_OK) {
+    free_state_buffers(&f);
+    return rc;
+  }
+  free_state_buffers(s);
+  *s = f;
   return MCB_OK;
 }
 
@@ -732,13 +761,21 @@ extern "C" mcb_status mcb_heat_forward(mcb_ctx *ctx, const mcb_heat_params *p, f
     s->ctx = ctx;
     ctx->heat = s;
   }
-  if (stream_supported(p->nx, p->ny, p->nz)) {
+  if (stream_supported(p->nx, p->ny, p->nz) || rows_supported(p->nx, p->ny, p->nz)) {
     if (!state_fits(s, p, damage, true)) MCB_TRY(stream_alloc(ctx, s, p, damage));
     MCB_TRY(stream_upload(ctx, s, p, T, Omega, heat_mean(T, (long long)p->nx * p->ny * p->nz)));
     if (p->lightsOn) MCB_TRY(stream_upload_q(ctx, s, p->dTdt_abs));
     MCB_TRY(sensor_buffers(ctx, s, p));
-    MCB_TRY(stream_step(ctx, s, p, s->sens, sensorTemps, maxMediaTemps, true));
-    return stream_download(ctx, s, T, Omega);
+    bool fits = true;
+    MCB_TRY(stream_step(ctx, s, p, s->sens, sensorTemps, maxMediaTemps, true, &fits));
+    if (fits) return stream_download(ctx, s, T, Omega);
+    // a long grid of many media: the factored stepper, on a state of its own (the streamed one stays
+    // for the next call)
+    if (!ctx->heatLong) {
+      ctx->heatLong = new mcb_heat_state();
+      ctx->heatLong->ctx = ctx;
+    }
+    s = ctx->heatLong;
   }
   if (!state_fits(s, p, damage, false)) MCB_TRY(state_alloc(ctx, s, p, damage));
   MCB_TRY(state_upload(ctx, s, p, T, Omega, heat_mean(T, s->L)));
@@ -756,7 +793,7 @@ extern "C" mcb_status mcb_heat_state_create(mcb_ctx *ctx, const mcb_heat_params 
   mcb_heat_state *s = new mcb_heat_state();
   s->ctx = ctx;
   mcb_status st;
-  if (stream_supported(p->nx, p->ny, p->nz)) {
+  if (stream_supported(p->nx, p->ny, p->nz) || rows_supported(p->nx, p->ny, p->nz)) {
     st = stream_alloc(ctx, s, p, Omega != nullptr);
     if (st == MCB_OK) st = stream_upload(ctx, s, p, T, Omega, heat_mean(T, (long long)p->nx * p->ny * p->nz));
     if (st == MCB_OK && p->lightsOn) st = stream_upload_q(ctx, s, p->dTdt_abs);
@@ -786,7 +823,10 @@ extern "C" mcb_status mcb_heat_state_step(mcb_heat_state *s, const mcb_heat_para
   if (s->streamed) {
     if (p->lightsOn && p->dTdt_abs) MCB_TRY(stream_upload_q(ctx, s, p->dTdt_abs));
     MCB_TRY(sensor_buffers(ctx, s, p));
-    return stream_step(ctx, s, p, s->sens, sensorTemps, maxMediaTemps, true);
+    bool fits = true;
+    MCB_TRY(stream_step(ctx, s, p, s->sens, sensorTemps, maxMediaTemps, true, &fits));
+    if (fits) return MCB_OK;
+    MCB_TRY(state_to_factored(ctx, s, p));
   }
   if (p->lightsOn && p->dTdt_abs)
     MCB_CUDA(ctx, cudaMemcpyAsync(s->Q, p->dTdt_abs, 4 * s->L, cudaMemcpyHostToDevice, ctx->stream));

@@ -26,10 +26,12 @@ struct StreamMaps {
 }  // namespace mcb
 
 // Device-resident stepper state: grids stay in HBM across calls. A state is either streamed
-// (heat_stream.cu: pitched grids, no stored factorisation) or factored (heat_adi.cu: dense grids
-// with the line factorisation stored per voxel, used by the adjoint and for axes over 512).
+// (heat_stream.cu, heat_rows.cu: pitched grids, no stored factorisation) or factored (heat_adi.cu:
+// dense grids with the line factorisation stored per voxel, used by the adjoint, and for axes over
+// 512 voxels where the coded-row passes do not take the grid).
 struct mcb_heat_state {
   bool streamed = false;
+  bool rowsOnly = false;  // streamed, with an axis over 512: coded-row passes only (no TMA-staged ones)
   mcb::StreamShape shape;
   mcb::StreamMaps *maps = nullptr;
   uint8_t *code = nullptr;
@@ -123,8 +125,9 @@ mcb_status stream_maps(mcb_ctx *ctx, mcb_heat_state *s);
 mcb_status stream_upload(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *p, const float *T, const float *Omega,
                          double base);
 mcb_status stream_upload_q(mcb_ctx *ctx, mcb_heat_state *s, const float *Q);
+// *fits false (nothing stepped): a rowsOnly state whose row coefficients do not fit the code tables.
 mcb_status stream_step(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *p, double *sens, double *sensorTemps,
-                       float *maxMediaTemps, bool graphs);
+                       float *maxMediaTemps, bool graphs, bool *fits = nullptr);
 mcb_status stream_download(mcb_ctx *ctx, mcb_heat_state *s, float *T, float *Omega);
 // T of a streamed state (pitched deviations) into a dense array of deviations, and back;
 // asynchronous.

@@ -1292,6 +1292,7 @@ struct StreamStepper {
   size_t xs = 0;
   bool colY = true, colZ = true;
   const mcb_heat_state *rows = nullptr;  // step with the coded-row passes (heat_rows.cu)
+  bool ready = true;                     // false: a rowsOnly state without row codes
 };
 
 // Per-call set-up of the streamed stepper on a state: the per-call tables (H = dt/2 c in FP32, as
@@ -1341,6 +1342,10 @@ mcb_status stream_setup(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *
       k.rows = s;
       return MCB_OK;
     }
+  }
+  if (s->rowsOnly) {
+    k.ready = false;
+    return MCB_OK;
   }
   h.uniX = s->uniX;
   h.uniY = s->uniY;
@@ -1427,13 +1432,15 @@ void stream_pitched_indices(const mcb_heat_state *s, const int *dense, int *pitc
 // Runs p->steps steps on the device-resident streamed state. Sensor and maximum outputs go to
 // host memory; `sens` is the device buffer of the sensor history ([nS x (steps + 1)] doubles).
 mcb_status stream_step(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *p, double *sens, double *sensorTemps,
-                       float *maxMediaTemps, bool graphs) {
+                       float *maxMediaTemps, bool graphs, bool *fits) {
   cudaStream_t st = ctx->stream;
   const StreamShape &S = s->shape;
   const long long L = (long long)S.nx * S.ny * S.nz, nt = p->steps;
   const int nM = p->nM, nS = p->nSensors;
   StreamStepper ks;
   MCB_TRY(stream_setup(ctx, s, p, sens, &ks));
+  if (fits) *fits = ks.ready;
+  if (!ks.ready) return MCB_OK;
   const StreamDev &h = ks.h;
   auto step = [&](cudaStream_t q) { stream_step_launch(ks, q); };
   MCB_CUDA(ctx, cudaEventRecord(ctx->ev0, st));

@@ -37,3 +37,50 @@ def test_media_varying_by_voxel(nM, hs, oracle_lib):
     case["hp"] = mexargs.heat_mex_params(M1, A, E, c, Q, True, hs, hp["tempSensorCornerIdxs"].ravel(),
                                          hp["tempSensorInterpWeights"], True, 8, 0.02)
     _check(case, oracle_lib)
+
+
+LONG = [(513, 5, 4), (700, 3, 5), (4, 513, 5), (5, 640, 4), (3, 1000, 4), (5, 4, 513), (6, 5, 641), (4, 3, 1024)]
+
+
+@pytest.mark.parametrize("shape", LONG, ids=lambda s: "x".join(map(str, s)))
+def test_long_axes(shape, oracle_lib):
+    """Axes over 512 voxels (32 rows per lane), heat-sinked faces on the odd ones."""
+    _check(heatcases.shaped(shape, seed=sum(shape), heatSinked=sum(shape) % 2, nt=5, dt_factor=15.0), oracle_lib)
+
+
+def _many_media(case, nM, dt, steps, hs=0):
+    """`case` with media varying voxel by voxel."""
+    from mcmatlab_b200 import mexargs, prep
+    rng = np.random.default_rng(nM)
+    M1 = rng.integers(1, nM + 1, case["n"]).astype(np.uint8)
+    c, Q = prep.calc_dTdt_arrays(rng.uniform(3.0, 4.2, nM), rng.uniform(0.002, 0.006, nM), 0.02, 0.02, 0.02,
+                                 40.0 * rng.random(case["n"]), 1.0, M1)
+    hp = case["hp"]
+    hp = mexargs.heat_mex_params(M1, np.full(nM, 7.6e66), np.full(nM, 4.48e5), c, Q, True, hs, hp["tempSensorCornerIdxs"].ravel(),
+                                 hp["tempSensorInterpWeights"], True, steps, dt)
+    return dict(case, hp=hp)
+
+
+def test_long_axis_of_many_media(oracle_lib):
+    """Too many row coefficients for the code tables on a grid the staged passes do not take either."""
+    _check(_many_media(heatcases.shaped((9, 7, 530), seed=5, nt=6), 24, 0.02, 6), oracle_lib)
+
+
+def test_long_state_outgrows_its_codes(oracle_lib):
+    """A resident state on a long axis whose codes fit at a small time step and not at a large one goes
+    on as a factored state, with its temperatures and damage, and back to small steps."""
+    from mcmatlab_b200 import native
+    from oracle import orc
+    base = heatcases.shaped((8, 9, 600), seed=6, nt=4)
+    calls = [_many_media(base, 3, dt, 4)["hp"] for dt in (1e-6, 2.0, 1e-6)]
+    T, O = base["T0"], base["Omega0"]
+    st = native.HeatState(T, O, calls[0], *base["n"])
+    try:
+        for hp in calls:
+            st.step(hp)
+            T, O, _, _ = orc.oracle_heat(T.astype(np.float32), O.astype(np.float32), hp, *base["n"])
+        Tg, Og = st.read()
+    finally:
+        st.close()
+    assert np.max(np.abs(Tg - T) / np.abs(T)) <= 3e-5  # 1e-5 per call
+    assert np.max(np.abs(Og - O)) <= 1e-4 * np.max(O)
