@@ -280,6 +280,12 @@ __global__ void __launch_bounds__(128) rows_code_kernel(const RowBuild b) {
   else line_codes<32>(b, canon, job, n, M, st, lineSink, live, G, out, outSt, med, b.px);
 }
 
+// Programmatic dependent launch: a pass lets the next one start as soon as all its blocks run
+// (pass_begin); the next one stages its codes and tables, which no pass writes, and waits for the
+// pass before it to complete (pass_wait) before it touches a grid.
+__device__ __forceinline__ void pass_begin() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+__device__ __forceinline__ void pass_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+
 __device__ __forceinline__ int code_at(const uint32_t *w, int k) { return (w[k >> 2] >> (8 * (k & 3))) & 255; }
 
 // Codes of one chunk, and of the row before it.
@@ -418,7 +424,9 @@ __global__ void __launch_bounds__(MAXT, MINB)
   __shared__ int4 sOff[32];  // offsets of the y-1, y+1, z-1, z+1 rows of each line (0: no neighbour)
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
   const int lines = h.ny * h.nz, line0 = blockIdx.x * 32;
+  pass_begin();
   if (line0 >= lines) {
+    pass_wait();
     record_sensors_p(h, *h.stepCounter);
     return;
   }
@@ -441,6 +449,7 @@ __global__ void __launch_bounds__(MAXT, MINB)
     const int z = line / h.ny, y = line - z * h.ny, sxy = (int)h.sxy;
     sOff[threadIdx.x] = make_int4(y > 0 ? -h.px : 0, y < h.ny - 1 ? h.px : 0, z > 0 ? -sxy : 0, z < h.nz - 1 ? sxy : 0);
   }
+  pass_wait();
   __syncthreads();
   // explicit part, 4 voxels of one line per thread and round
   for (int i = threadIdx.x; i < items; i += nt) {
@@ -544,6 +553,7 @@ __global__ void __launch_bounds__(MAXT, MINB) rows_col_kernel(const StreamDev h,
   __shared__ float2 sF[kCodes], sB[kCodes];  // {a, 1 / b'}, {c / b', 1 / b'}
   __shared__ int sMed[ZP ? kCodes : 1];
   __shared__ unsigned int mloc[ZP ? 256 : 1];
+  pass_begin();
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
   const int n = ZP ? h.nz : h.ny;
   const int xTiles = (h.nx + 31) >> 5;
@@ -573,11 +583,7 @@ __global__ void __launch_bounds__(MAXT, MINB) rows_col_kernel(const StreamDev h,
       for (int k = 0; k < K; k++) dst[k] = k < cnt ? *row(p, st, k) : 0.f;
     }
   };
-  fetch(r, h.A + base);
   const int one = ZP && col ? rd.zMed[(o * G + w) * h.px + x] : 255;
-  float t[ZP ? K : 1];
-  float *p = (ZP ? h.T : h.A) + base;
-  if constexpr (ZP) fetch(t, p);
   {
     const float4 *tab = rd.tab + (ZP ? 3 : 2) * kCodes;
     for (int k = threadIdx.x; k < kCodes; k += blockDim.x) {
@@ -590,6 +596,11 @@ __global__ void __launch_bounds__(MAXT, MINB) rows_col_kernel(const StreamDev h,
       }
     }
   }
+  pass_wait();
+  fetch(r, h.A + base);
+  float t[ZP ? K : 1];
+  float *p = (ZP ? h.T : h.A) + base;
+  if constexpr (ZP) fetch(t, p);
   __syncthreads();
   const bool uni = __all_sync(0xffffffffu, cw.same());
   solve_rows<K>(r, cw, sF, sB, csums, w, l, G, uni);
@@ -674,6 +685,21 @@ size_t col_sums(int n) { return (size_t)2 * rc_warps(n) * 32 * sizeof(float2); }
 int x_quads(int nx) { return (nx + 3) / 4; }
 size_t x_tile(int nx) { return (size_t)x_quads(nx) * 128 * 4 * 2 + col_sums(nx); }
 
+template <typename... P, typename... A>
+void pass_launch(void (*kern)(P...), int grid, int threads, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kern, args...);  // a failure is found by the caller's cudaGetLastError
+}
+
 // Block classes of the Y and Z passes: up to 8 warps (128 rows), 13 (208), 20 (320), 32 (512), and
 // with 32 rows per lane 20 warps (640) or 32 (1024).
 template <bool ZP>
@@ -681,14 +707,14 @@ void col_launch(const StreamDev &h, const RowDev &rd, int n, int grid, cudaStrea
   const int G = rc_warps(n);
   const size_t sm = col_sums(n);
   if (rc_rows(n) == 16) {
-    if (G <= 8) rows_col_kernel<16, ZP, 256, ZP ? 3 : 4><<<grid, 32 * G, sm, st>>>(h, rd, G);
-    else if (G <= 13) rows_col_kernel<16, ZP, 416, 2><<<grid, 32 * G, sm, st>>>(h, rd, G);
-    else if (G <= 20) rows_col_kernel<16, ZP, 640, ZP ? 1 : 2><<<grid, 32 * G, sm, st>>>(h, rd, G);
-    else rows_col_kernel<16, ZP, 1024, 1><<<grid, 32 * G, sm, st>>>(h, rd, G);
+    if (G <= 8) pass_launch(rows_col_kernel<16, ZP, 256, ZP ? 3 : 4>, grid, 32 * G, sm, st, h, rd, G);
+    else if (G <= 13) pass_launch(rows_col_kernel<16, ZP, 416, 2>, grid, 32 * G, sm, st, h, rd, G);
+    else if (G <= 20) pass_launch(rows_col_kernel<16, ZP, 640, ZP ? 1 : 2>, grid, 32 * G, sm, st, h, rd, G);
+    else pass_launch(rows_col_kernel<16, ZP, 1024, 1>, grid, 32 * G, sm, st, h, rd, G);
   } else if (G <= 20) {
-    rows_col_kernel<32, ZP, 640, 1><<<grid, 32 * G, sm, st>>>(h, rd, G);
+    pass_launch(rows_col_kernel<32, ZP, 640, 1>, grid, 32 * G, sm, st, h, rd, G);
   } else {
-    rows_col_kernel<32, ZP, 1024, 1><<<grid, 32 * G, sm, st>>>(h, rd, G);
+    pass_launch(rows_col_kernel<32, ZP, 1024, 1>, grid, 32 * G, sm, st, h, rd, G);
   }
 }
 
@@ -793,7 +819,7 @@ void rows_step_launch(const mcb_heat_state *s, const StreamDev &h, cudaStream_t 
   const long long lines = (long long)S.ny * S.nz;
   // i / quads = umulhi(i, ceil(2^32 / quads)) for i < 32 quads <= 2^13
   const uint32_t rcp = quads > 1 ? (uint32_t)((0x100000000ull + quads - 1) / quads) : 0u;
-  x_kernel(S.nx, [&](auto kern) { kern<<<(int)((lines + 31) / 32) + (h.nS > 0), 32 * G, x_tile(S.nx), q>>>(h, rd, G, quads, rcp); });
+  x_kernel(S.nx, [&](auto kern) { pass_launch(kern, (int)((lines + 31) / 32) + (h.nS > 0), 32 * G, x_tile(S.nx), q, h, rd, G, quads, rcp); });
   const int xTiles = (S.nx + 31) / 32;
   col_launch<false>(h, rd, S.ny, xTiles * S.nz, q);
   col_launch<true>(h, rd, S.nz, xTiles * S.ny, q);

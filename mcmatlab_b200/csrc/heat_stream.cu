@@ -1446,7 +1446,10 @@ mcb_status stream_step(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *p
   MCB_CUDA(ctx, cudaEventRecord(ctx->ev0, st));
   const int chunk = 16;
   long long done = 0;
-  if (graphs && nt >= chunk) {
+  // the coded passes are launched one by one: programmatic dependent launch hides their launch latency
+  // (100^3: 20.9 us per step against 21.9 from a graph of 16 steps; a call of 20 steps on 31 x 27 x 40 voxels
+  // saves the graph's 100 us)
+  if (graphs && !ks.rows && nt >= chunk) {
     cudaGraph_t graph;
     cudaGraphExec_t exec;
     MCB_CUDA(ctx, cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
