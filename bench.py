@@ -252,7 +252,7 @@ def run_ours(args):
                      # L2-resident
                      "traffic": HEAT_STEP_DRAM_BYTES, "traffic_note": "ncu cold-cache capture, bytes per DG-ADI step",
                      "algorithmic_bytes_per_voxel_update": bytes_per_update,
-                     "kernel": "DG-ADI step (sx_kernel + scol_kernel<y> + scol_kernel<z>)"},
+                     "kernel": "DG-ADI step (rows_x_kernel + rows_col_kernel<y> + rows_col_kernel<z>)"},
         "light_off": {"workload": "same state and dt, light off (the cooling phase of the schedule)",
                       "value": float(L) * args.nt / (off_ms / 1e3), "unit": "voxel-updates/s", "ms_per_step": off_ms,
                       "steps": len(off_times),
