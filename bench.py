@@ -288,7 +288,10 @@ def run_ours(args):
     if args.lbfgs and ws == 1:
         res["lbfgs"] = lbfgs_measure(dev, args.c3_packets, args.c3_grid)
     if rank == 0:
-        if args.cpu_baseline:
+        missing = reference_missing() if args.cpu_baseline else None
+        if missing:
+            res["cpu_baseline"] = {"unavailable": missing}
+        elif args.cpu_baseline:
             res["cpu_baseline"] = cpu_baseline(args, sample_steps=args.ref_nt)
             res["mc"]["cpu_baseline"] = res["cpu_baseline"].pop("mc")
             c4 = res["cpu_baseline"].pop("heat_c4")
@@ -424,6 +427,15 @@ def lbfgs_measure(dev, packets, n):
 REF_MC_PACKETS = 1e6
 
 
+def reference_missing():
+    """Why the reference's libraries cannot be timed on this machine, or None where they were built."""
+    from oracle import ref
+    for lib in ("libref_mc.so", "libref_heat.so"):
+        if not os.path.exists(os.path.join(ref.REF_DIR, lib)):
+            return "oracle/_ref/%s is not built (the reference's sources are needed for it)" % lib
+    return None
+
+
 def reference_setup(timings=None):
     from oracle import ref
     m = configs.standard_tissue_cube(n=N_GRID, nPhotons=REF_MC_PACKETS, seed=1)
@@ -498,6 +510,10 @@ def run_reference(args):
     if rank != 0:
         return
     from oracle import ref
+    missing = reference_missing()
+    if missing:
+        print(json.dumps({"impl": "reference", "unavailable": missing}), flush=True)
+        return
     m, NA = reference_setup()
     th, c, Q, dt = build_heat_inputs(NA, m)
     hp = mexargs.heat_mex_params(th["M"], th["A"], th["E"], c, Q, True, 0, None, None, True, args.ref_nt, dt)
