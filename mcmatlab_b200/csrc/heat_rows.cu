@@ -478,7 +478,7 @@ __global__ void __launch_bounds__(MAXT, MINB)
       if (!same) e = sYZ[c >> 24];
       g.w = lap(t.w, ym.w, yp.w, zm.w, zp.w);
       if (h.Q) {
-        // (the x entry of heat-sinked voxels and padding, 0, removes the source again in the solve)
+        // (the x entry of heat-sinked voxels and padding, 0, drops the source again in the solve)
         const float4 q = *reinterpret_cast<const float4 *>(h.Q + v);
         g.x = fmaf(h.dt, q.x, g.x);
         g.y = fmaf(h.dt, q.y, g.y);
@@ -504,15 +504,18 @@ __global__ void __launch_bounds__(MAXT, MINB)
     const bool uni = __all_sync(0xffffffffu, cw.same());
     auto at = [&](int k) { return s * 32 + k * 32 + (l ^ (((s >> 2) + (k & ~15) / 4) & 31) ^ ((k >> 2) & 3)); };
     float r[K];
+    // heat-sinked rows and padding (e.w 0) take no right-hand side, by a select and not a product: their
+    // source may hold anything, and a product would turn an infinity into NaN
     float tl = s > 0 ? sT[xt(s - 1, l)] : 0.f, t = sT[at(0)];
     if (uni && rows == K) {
       const float4 e = sE[cw.at(0)];
+      const bool free = e.w != 0.f;
 #pragma unroll
       for (int k = 0; k < K; k++) {
         float tr;
         if (k + 1 < K) tr = sT[at(k + 1 < K ? k + 1 : k)];
         else tr = s + K < 4 * quads ? sT[xt(s + K, l)] : 0.f;
-        r[k] = fmaf(2.f, e.x * (tl - t) + e.y * (tr - t), e.w * sR[at(k)]);
+        r[k] = fmaf(2.f, e.x * (tl - t) + e.y * (tr - t), free ? sR[at(k)] : 0.f);
         tl = t;
         t = tr;
       }
@@ -523,7 +526,7 @@ __global__ void __launch_bounds__(MAXT, MINB)
         if (k < rows) {
           const float4 e = sE[cw.at(k)];
           const float tr = k + 1 < rows || s + K < 4 * quads ? sT[xt(s + k + 1, l)] : 0.f;
-          r[k] = fmaf(2.f, e.x * (tl - t) + e.y * (tr - t), e.w * sR[at(k)]);
+          r[k] = fmaf(2.f, e.x * (tl - t) + e.y * (tr - t), e.w != 0.f ? sR[at(k)] : 0.f);
           tl = t;
           t = tr;
         }
