@@ -1,5 +1,6 @@
 """The heat stepper at the limits of its inputs: sources that are not finite on heat-sinked faces
-(held voxels take no source)."""
+(held voxels take no source), and line matrices far from diagonal dominance (pivots that settle
+slowly)."""
 import numpy as np
 import pytest
 
@@ -28,3 +29,25 @@ def test_source_on_sinked_faces_is_ignored(shape, steps, bad, oracle_lib):
     for a, b in zip(*runs):
         np.testing.assert_array_equal(a, b)
     np.testing.assert_array_equal(runs[1][0][face], case["T0"][face])
+
+
+@pytest.mark.parametrize("axis", [0, 1, 2])
+@pytest.mark.parametrize("H", [60.0, 300.0, 1000.0])
+def test_uniform_heating_of_a_stiff_line(axis, H):
+    """An insulated block of one medium under a uniform source warms up uniformly, by dt Q per step,
+    whatever its couplings. With a coupling of H = dt/2 c the pivots settle over about 10 sqrt(H) rows
+    and a pivot error is amplified H-fold: FP32 pivots rounded from converged FP64 ones leave at most
+    1.5e-6 of the rise (FP32 line solves emulated on the CPU for these H), pivots frozen at the first two
+    that round alike 1.2e-5 at H = 300 and 5e-5 at H = 1000. Bound: 5e-6."""
+    from mcmatlab_b200 import mexargs, native
+    shape = [5, 5, 5]
+    shape[axis] = 500
+    dt, Q, steps = 0.1, 250.0, 4
+    c = np.full((1, 1, 3), 0.5, np.float32)
+    c[0, 0, axis] = 2 * H / dt
+    T0 = np.full(shape, 20.0, np.float32, order="F")
+    hp = mexargs.heat_mex_params(np.ones(shape, np.uint8), [0.0], [0.0], c, np.full(shape, Q, np.float32), True, 0, None,
+                                 None, True, steps, dt)
+    T, _, _, _ = native.heat_forward(T0, None, hp, *shape)
+    rise = steps * dt * Q
+    assert np.max(np.abs(T.astype(np.float64) - 20.0 - rise)) <= 5e-6 * rise
