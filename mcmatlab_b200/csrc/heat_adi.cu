@@ -399,11 +399,8 @@ size_t x_smem(int nx) { return x_smem_lines(nx, x_lines(nx)); }
 
 template <int TW>
 mcb_status setup_yz(mcb_ctx *ctx, int ny, int nz) {
-  MCB_CUDA(ctx, cudaFuncSetAttribute(pass_yz_kernel<TW, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)yz_smem(TW, ny)));
-  MCB_CUDA(ctx, cudaFuncSetAttribute(pass_yz_kernel<TW, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)yz_smem(TW, nz)));
-  return MCB_OK;
+  MCB_TRY(smem_allow(ctx, (const void *)pass_yz_kernel<TW, false>, yz_smem(TW, ny)));
+  return smem_allow(ctx, (const void *)pass_yz_kernel<TW, true>, yz_smem(TW, nz));
 }
 
 template <int TW>
@@ -724,7 +721,7 @@ mcb_status heat_stepper(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *
   MCB_CUDA(ctx, cudaMemsetAsync(s->step, 0, 16, st));
   if (s->dOm) MCB_CUDA(ctx, cudaMemsetAsync(s->dOm, 0, 4 * (size_t)L, st));
   k.smemX = x_smem((int)nx);
-  MCB_CUDA(ctx, cudaFuncSetAttribute(pass_x_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.smemX));
+  MCB_TRY(smem_allow(ctx, (const void *)pass_x_kernel, k.smemX));
   k.tw = s->tw;
   if (k.tw == 32) MCB_TRY(setup_yz<32>(ctx, (int)ny, (int)nz));
   else if (k.tw == 16) MCB_TRY(setup_yz<16>(ctx, (int)ny, (int)nz));

@@ -744,11 +744,8 @@ void adj_col_launch(const AdjDev &a, int n, int grid, cudaStream_t st) {
 
 template <int TW>
 mcb_status adj_setup_yz(mcb_ctx *ctx, int ny, int nz) {
-  MCB_CUDA(ctx, cudaFuncSetAttribute(adj_solve_yz_kernel<TW, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)(adj_yz_tile_bytes<TW>(ny) + 64)));
-  MCB_CUDA(ctx, cudaFuncSetAttribute(adj_solve_yz_kernel<TW, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)(adj_yz_tile_bytes<TW>(nz) + 64)));
-  return MCB_OK;
+  MCB_TRY(smem_allow(ctx, (const void *)adj_solve_yz_kernel<TW, false>, adj_yz_tile_bytes<TW>(ny) + 64));
+  return smem_allow(ctx, (const void *)adj_solve_yz_kernel<TW, true>, adj_yz_tile_bytes<TW>(nz) + 64);
 }
 
 template <int TW>
@@ -919,7 +916,8 @@ extern "C" mcb_status mcb_heat_adjoint(mcb_ctx *ctx, const mcb_heat_params *pin,
   const int tw = s.tw;
   const int nx = p.nx, ny = p.ny, nz = p.nz;
   const size_t smemX = (size_t)a.h.xl * 16 * (nx + 1) + 64;
-  ADJ_CUDA(cudaFuncSetAttribute(adj_solve_x_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemX));
+  rc = smem_allow(ctx, (const void *)adj_solve_x_kernel, smemX);
+  if (rc != MCB_OK) return fail(rc);
   if (tw == 32) rc = adj_setup_yz<32>(ctx, ny, nz);
   else if (tw == 16) rc = adj_setup_yz<16>(ctx, ny, nz);
   else rc = adj_setup_yz<8>(ctx, ny, nz);
@@ -937,7 +935,8 @@ extern "C" mcb_status mcb_heat_adjoint(mcb_ctx *ctx, const mcb_heat_params *pin,
   a.zChunk = adj_z_chunk(tilesZ, nz, ctx->num_sms * (1024 / kZCN));
   const dim3 gridZ((nx + kZX - 1) / kZX, (ny + kZY - 1) / kZY, (nz + a.zChunk - 1) / a.zChunk);
   const size_t smemZ = (size_t)3 * nM * nM * (8 + 4);
-  ADJ_CUDA(cudaFuncSetAttribute(adj_assemble_z_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemZ));
+  rc = smem_allow(ctx, (const void *)adj_assemble_z_kernel, smemZ);
+  if (rc != MCB_OK) return fail(rc);
   a.dQinX = gridXL != 0;
 
   // The forward sweeps (checkpoints, segment recomputation) step a streamed state where the grid

@@ -812,10 +812,7 @@ mcb_status rows_build(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *p,
   const long long most = std::max({(long long)S.ny * S.nz * (S.px / 4), (long long)S.px * S.nz, (long long)S.px * S.ny, (long long)S.ny * S.nz + 31});
   rows_code_kernel<<<dim3((unsigned)((most + 127) / 128), 4), 128, 0, st>>>(b);
   MCB_CUDA(ctx, cudaGetLastError());
-  MCB_TRY(x_kernel(S.nx, [&](auto kern) -> mcb_status {
-    MCB_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)x_tile(S.nx)));
-    return MCB_OK;
-  }));
+  MCB_TRY(x_kernel(S.nx, [&](auto kern) { return smem_allow(ctx, (const void *)kern, x_tile(S.nx)); }));
   int over = 0;
   MCB_CUDA(ctx, cudaMemcpyAsync(&over, b.over, 4, cudaMemcpyDeviceToHost, st));
   MCB_CUDA(ctx, cudaStreamSynchronize(st));

@@ -1067,13 +1067,12 @@ size_t yz_smem(int n, bool z) { return 2 * (size_t)yz_layout(n, z).stage + 64 + 
 
 template <int K, int G>
 mcb_status x_attr(mcb_ctx *ctx, size_t bytes) {
-  MCB_CUDA(ctx, cudaFuncSetAttribute(sx_kernel<K, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-  return MCB_OK;
+  return smem_allow(ctx, (const void *)sx_kernel<K, G>, bytes);
 }
 
 template <int K, int G, bool Z>
 mcb_status yz_attr(mcb_ctx *ctx, size_t bytes, int *blocksPerSm) {
-  MCB_CUDA(ctx, cudaFuncSetAttribute(syz_kernel<K, G, Z>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  MCB_TRY(smem_allow(ctx, (const void *)syz_kernel<K, G, Z>, bytes));
   MCB_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocksPerSm, syz_kernel<K, G, Z>, 16 * G, bytes));
   return MCB_OK;
 }
@@ -1094,7 +1093,7 @@ size_t col_smem(int n, bool z) {
 template <int K, bool Z, int MAXT>
 mcb_status col_attr(mcb_ctx *ctx, int n, int *bps) {
   const size_t sm = col_smem(n, Z);
-  MCB_CUDA(ctx, cudaFuncSetAttribute(scol_kernel<K, Z, MAXT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  MCB_TRY(smem_allow(ctx, (const void *)scol_kernel<K, Z, MAXT>, sm));
   MCB_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(bps, scol_kernel<K, Z, MAXT>, 32 * col_warps(n), sm));
   return MCB_OK;
 }

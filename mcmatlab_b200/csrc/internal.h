@@ -37,6 +37,7 @@ struct mcb_ctx {
   std::string gpuName;
   std::map<int, mcb_mc_launch> tuned;
   mcb_mc_launch force{0, 0};
+  std::map<const void *, size_t> smemMost;  // kernels whose shared-memory limit is set (smem_allow)
 };
 
 namespace mcb {
@@ -85,6 +86,27 @@ void tune_file_load(mcb_ctx *ctx);
     mcb_status _s = (expr);           \
     if (_s != MCB_OK) return _s;      \
   } while (0)
+
+// Lets a block of `kernel` have `bytes` of dynamic shared memory. The limit is a property of the device
+// that all its contexts share, so it is always set to the same value, the most a block can have beside the
+// kernel's static part: a limit of one call's size could be lowered by another thread's call between
+// this one's set and its launch, which then fails. (What a launch takes is the size it is given.) Set
+// once per context and kernel.
+inline mcb_status smem_allow(mcb_ctx *ctx, const void *kernel, size_t bytes) {
+  size_t &most = ctx->smemMost[kernel];
+  if (!most) {
+    cudaFuncAttributes fa;
+    MCB_CUDA(ctx, cudaFuncGetAttributes(&fa, kernel));
+    int optin = 0;
+    MCB_CUDA(ctx, cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
+    const int free = optin - (int)fa.sharedSizeBytes;
+    MCB_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, free));
+    most = (size_t)free;
+  }
+  if (bytes > most)
+    return set_error(ctx, MCB_ECUDA, "a block needs %zu bytes of shared memory, more than its limit of %zu", bytes, most);
+  return MCB_OK;
+}
 
 // Buffer slots used by the pool.
 enum PoolSlot {

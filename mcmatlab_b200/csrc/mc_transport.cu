@@ -1010,7 +1010,7 @@ mcb_status launch_transport(mcb_ctx *ctx, Arena &ar, const std::vector<Inst> &in
                                : feat & kFeatCrit ? transport_kernel<false, kFeatAll>
                                : feat             ? transport_kernel<false, kFeatTime>
                                                   : transport_kernel<false, 0>;
-  if (grad) MCB_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dynSmem));
+  if (grad) MCB_TRY(smem_allow(ctx, (const void *)kernel, dynSmem));
   int blocksPerSm = 0;
   MCB_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocksPerSm, kernel, 256, dynSmem));
   if (blocksPerSm < 1) blocksPerSm = 1;

@@ -234,7 +234,7 @@ mcb_status axis_launch(mcb_ctx *ctx, const float *in, float *out, const float *C
   const int groups = padded(n) / 8, most = 256 / (TL / 4), rounds = (groups + most - 1) / most;
   const int threads = ((groups + rounds - 1) / rounds * (TL / 4) + 31) & ~31;  // whole warps
   const size_t sm = (size_t)n * TL * 4 + 32 * (size_t)(threads / (TL / 4) * 8) * 4;
-  MCB_CUDA(ctx, cudaFuncSetAttribute(axis_kernel<TL, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  MCB_TRY(smem_allow(ctx, (const void *)axis_kernel<TL, EPI>, sm));
   axis_kernel<TL, EPI><<<dim3((unsigned)((lines + TL - 1) / TL), 3), threads, sm, ctx->stream>>>(in, out, CT, padded(n), nx, ny, nz, axis,
                                                                                    lam, s, M1, riClass, cls);
   MCB_CUDA(ctx, cudaGetLastError());

@@ -1,6 +1,9 @@
 """The heat stepper at the limits of its inputs: sources that are not finite on heat-sinked faces
-(held voxels take no source), and line matrices far from diagonal dominance (pivots that settle
-slowly)."""
+(held voxels take no source), line matrices far from diagonal dominance (pivots that settle slowly),
+and contexts of several threads that step grids of one launch class at the same time."""
+import ctypes
+import threading
+
 import numpy as np
 import pytest
 
@@ -51,3 +54,43 @@ def test_uniform_heating_of_a_stiff_line(axis, H):
     T, _, _, _ = native.heat_forward(T0, None, hp, *shape)
     rise = steps * dt * Q
     assert np.max(np.abs(T.astype(np.float64) - 20.0 - rise)) <= 5e-6 * rise
+
+
+@pytest.mark.parametrize("steps", [3, 4])
+def test_threads_share_a_launch_class(steps, oracle_lib):
+    """Two contexts, one per thread, step grids whose passes are the same kernels with different amounts
+    of shared memory. Every call succeeds and gives what it gives alone."""
+    from mcmatlab_b200 import abi, native
+    lib = native.lib()
+    fp = ctypes.POINTER(ctypes.c_float)
+    cases = [heatcases.shaped(s, seed=3, nt=steps, with_damage=False) for s in ((126, 40, 40), (18, 40, 40))]
+    alone = [native.heat_forward(c["T0"], None, c["hp"], *c["n"])[0] for c in cases]
+    errors = []
+
+    def work(k):
+        ctx = ctypes.c_void_p()
+        assert lib.mcb_ctx_create(0, ctypes.byref(ctx)) == 0
+        try:
+            hb = abi.HeatParamBuffers(*cases[k]["n"], cases[k]["hp"])
+            T0 = np.ascontiguousarray(cases[k]["T0"].reshape(-1, order="F"))
+            sens = np.zeros(max(hb.nS * (steps + 1), 1))
+            mx = np.zeros(hb.nM, np.float32)
+            for rep in range(400):
+                T = T0.copy()
+                st = lib.mcb_heat_forward(ctx, ctypes.byref(hb.params), T.ctypes.data_as(fp), ctypes.cast(None, fp),
+                                          sens.ctypes.data_as(ctypes.POINTER(ctypes.c_double)), mx.ctypes.data_as(fp))
+                if st != 0:
+                    errors.append((k, rep, lib.mcb_last_error(ctx).decode()))
+                    return
+                if not np.array_equal(T.reshape(cases[k]["n"], order="F"), alone[k]):
+                    errors.append((k, rep, "differs"))
+                    return
+        finally:
+            lib.mcb_ctx_destroy(ctx)
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
