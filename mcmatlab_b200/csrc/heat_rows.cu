@@ -90,26 +90,54 @@ __global__ void rows_init_kernel(unsigned long long *keys, float4 *tab, int *med
   if (j == 0 && t == 0) *over = 0;
 }
 
-// Code of `key` in table j: found, or inserted with its entry by the thread that wins the slot.
-__device__ __forceinline__ int row_code(const RowBuild &b, int j, unsigned long long key, float4 e, int med) {
-  unsigned long long *keys = b.keys + j * kCodes;
-  unsigned long long hsh = key * 0x9E3779B97F4A7C15ull;
-  int s = 1 + (int)((hsh >> 40) % 255u);
-  for (int t = 0; t < 255; t++) {
-    unsigned long long cur = *(volatile unsigned long long *)(keys + s);
-    if (cur == 0ull) {
-      cur = atomicCAS(keys + s, 0ull, key);
-      if (cur == 0ull) {
-        b.tab[j * kCodes + s] = e;
-        if (j == 3) b.med[s] = med;
-        return s;
+// Whether a table has overflowed: the call will not use the codes, so every walk ends.
+__device__ __forceinline__ bool rows_over(const RowBuild &b) { return *(volatile int *)b.over != 0; }
+
+// Code of `key`, the number of its slot: found, or entered by the thread that wins the slot. What a lookup
+// costs is the latency of its dependent loads: the slots are read four at a time, group after group from the
+// key's own, and every search ends once one has found a table full.
+__device__ __forceinline__ int probe_code(unsigned long long *keys, float4 *tab, int *med, int *over, unsigned long long key, float4 e,
+                                          int medium) {
+  const unsigned long long hsh = key * 0x9E3779B97F4A7C15ull;
+  int g = (int)((hsh >> 40) & (kCodes / 4 - 1));
+  for (int t = 0; t < kCodes / 4; t++, g = (g + 1) & (kCodes / 4 - 1)) {
+    const unsigned long long *p = keys + 4 * g;
+    unsigned long long cur[4];
+    asm volatile("ld.volatile.global.v2.u64 {%0, %1}, [%2];" : "=l"(cur[0]), "=l"(cur[1]) : "l"(p));
+    asm volatile("ld.volatile.global.v2.u64 {%0, %1}, [%2];" : "=l"(cur[2]), "=l"(cur[3]) : "l"(p + 2));
+    if (*(volatile int *)over) return 0;
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const int s = 4 * g + q;
+      if (cur[q] == 0ull) {
+        cur[q] = atomicCAS(keys + s, 0ull, key);
+        if (cur[q] == 0ull) {
+          tab[s] = e;
+          if (med) med[s] = medium;
+          return s;
+        }
       }
+      if (cur[q] == key) return s;
     }
-    if (cur == key) return s;
-    s = s == 255 ? 1 : s + 1;
   }
-  *b.over = 1;
+  *(volatile int *)over = 1;
   return 0;
+}
+
+// One search per key of the lanes that come here together: the lines of a warp mostly hold the same rows, and
+// all warps of the first wave look for the same few keys at once. (A function of its own: inlined at every
+// row of the unrolled walks it takes their registers.)
+__device__ __noinline__ int find_code(unsigned long long *keys, float4 *tab, int *med, int *over, unsigned long long key, float4 e,
+                                      int medium) {
+  const unsigned int group = __match_any_sync(__activemask(), key);
+  const int leader = __ffs(group) - 1;
+  int code = 0;
+  if ((int)(threadIdx.x & 31) == leader) code = probe_code(keys, tab, med, over, key, e, medium);
+  return __shfl_sync(group, code, leader);
+}
+
+__device__ __forceinline__ int row_code(const RowBuild &b, int j, unsigned long long key, float4 e, int med) {
+  return find_code(b.keys + j * kCodes, b.tab + j * kCodes, j == 3 ? b.med : nullptr, b.over, key, e, med);
 }
 
 // The pivot recurrence along one line, row by row.
@@ -170,6 +198,7 @@ __device__ __forceinline__ void line_codes(const RowBuild &b, const uint8_t *can
   RowWalk w;
   int mp = 0, mr = live ? M[0] : 0;  // mr: the row's real medium
   for (int g = 0; g < G; g++) {
+    const bool over = rows_over(b);
     uint32_t word[4 * NW];
 #pragma unroll
     for (int q = 0; q < 4 * NW; q++) word[q] = 0u;
@@ -179,6 +208,7 @@ __device__ __forceinline__ void line_codes(const RowBuild &b, const uint8_t *can
       int nxt[K];
 #pragma unroll
       for (int k = 0; k < K; k++) nxt[k] = s + k + 1 < n ? M[(s + k + 1) * st] : 0;
+      if (over) return;
 #pragma unroll
       for (int k = 0; k < K; k++) {
         const int i = s + k;
@@ -209,6 +239,7 @@ __global__ void __launch_bounds__(128) rows_code_kernel(const RowBuild b) {
   if (job == 3) {
     const int quads = b.px / 4;
     if (t >= (long long)b.ny * b.nz * quads) return;
+    const bool over = rows_over(b);
     const int x4 = (int)(t % quads) * 4;
     const long long line = t / quads;
     const int y = (int)(line % b.ny), z = (int)(line / b.ny);
@@ -221,6 +252,7 @@ __global__ void __launch_bounds__(128) rows_code_kernel(const RowBuild b) {
     uint32_t nw[4];
 #pragma unroll
     for (int s = 0; s < 4; s++) nw[s] = f[s] ? *reinterpret_cast<const uint32_t *>(row + st[s]) : 0u;
+    if (over) return;
     unsigned long long lastKey = 0ull;
     int last = 0;
     uint32_t code = 0u;

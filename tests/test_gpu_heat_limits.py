@@ -1,8 +1,10 @@
 """The heat stepper at the limits of its inputs: sources that are not finite on heat-sinked faces
 (held voxels take no source), line matrices far from diagonal dominance (pivots that settle slowly),
-and contexts of several threads that step grids of one launch class at the same time."""
+contexts of several threads that step grids of one launch class at the same time, and media whose row
+coefficients do not fit the code tables."""
 import ctypes
 import threading
+import time
 
 import numpy as np
 import pytest
@@ -94,3 +96,48 @@ def test_threads_share_a_launch_class(steps, oracle_lib):
     for t in threads:
         t.join()
     assert not errors, errors
+
+
+def voxelwise(shape, nM, steps, dt_factor=1.5, seed=1, hs=0):
+    """A case whose medium changes from voxel to voxel."""
+    from mcmatlab_b200 import mexargs, prep
+    rng = np.random.default_rng(seed)
+    M1 = rng.integers(1, nM + 1, shape).astype(np.uint8)
+    TC, VHC, d = rng.uniform(0.002, 0.006, nM), rng.uniform(3.0, 4.2, nM), 0.01
+    c, Q = prep.calc_dTdt_arrays(VHC, TC, d, d, d, 40.0 * rng.random(shape), 1.0, M1)
+    dt = dt_factor * float(np.min(VHC / TC)) * d * d / 6
+    A, E = np.where(np.arange(nM) % 2, 7.6e66, 0.0), np.where(np.arange(nM) % 2, 4.48e5, 0.0)
+    hp = mexargs.heat_mex_params(M1, A, E, c, Q, True, hs, None, None, True, steps, dt)
+    T0 = np.asfortranarray((50 + 10 * rng.random(shape)).astype(np.float32))
+    return dict(T0=T0, Omega0=np.zeros(shape, np.float32, order="F"), hp=hp, n=shape)
+
+
+def triples(M):
+    """Distinct (previous, own, next) media of the rows along each axis: at least that many row
+    coefficients, so more than 255 along any axis cannot be coded."""
+    out = []
+    for ax in range(3):
+        m = np.moveaxis(np.asarray(M).astype(np.int64), ax, 0)
+        out.append(np.unique((m[:-2] * 256 + m[1:-1]) * 256 + m[2:]).size)
+    return out
+
+
+def test_row_code_overflow_is_cheap():
+    """Four steps on a resident state whose row coefficients overflow the code tables find that out in less
+    than the time of a call of three (which does not try): the bound leaves room for a few fold, the full
+    search of every failing row was about 15-fold."""
+    from mcmatlab_b200 import native
+    case = voxelwise((100, 100, 100), 24, 4)
+    assert max(triples(case["hp"]["M"])) > 255
+    best = {}
+    for steps in (3, 4):
+        hp = dict(case["hp"], steps=float(steps))
+        st = native.HeatState(case["T0"], case["Omega0"], hp, *case["n"])
+        try:
+            for _ in range(8):
+                t = time.perf_counter()
+                st.step(hp)
+                best[steps] = min(best.get(steps, 1.0), time.perf_counter() - t)
+        finally:
+            st.close()
+    assert best[4] <= 3 * best[3], best
