@@ -45,6 +45,11 @@ struct mcb_heat_state {
   float *H = nullptr;
   float4 *Hd = nullptr;
   int codeHs = -1;
+  // time step, boundary type and coefficients with which the row codes of the state's media did not fit
+  // (everything else they follow from stays with the state); noCodesHs -1: none known
+  int noCodesHs = -1;
+  double noCodesDt = 0.0;
+  std::vector<float> noCodesC;
   bool qValid = false;
   int lastW = 0;
   mcb_ctx *ctx = nullptr;

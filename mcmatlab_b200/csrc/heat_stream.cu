@@ -41,6 +41,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <mutex>
 #include <vector>
 
@@ -1267,6 +1268,7 @@ mcb_status stream_upload(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params 
   if (s->Om && Omega) MCB_CUDA(ctx, cudaMemcpyAsync(s->Om, Omega, 4 * L, cudaMemcpyHostToDevice, st));
   MCB_CUDA(ctx, cudaGetLastError());
   s->codeHs = (int)(p->heatBoundaryType != 0);
+  s->noCodesHs = -1;
   s->qValid = false;
   return MCB_OK;
 }
@@ -1337,8 +1339,19 @@ mcb_status stream_setup(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *
   // The codes cost about three of the steps they speed up (100^3: 60 us against 20 saved per step,
   // 300x300x200: 0.45 ms against 0.17), so shorter calls take the staged passes.
   if (s->rowX && (s->rowsOnly || p->steps >= 4)) {
-    bool coded = false;
-    MCB_TRY(rows_build(ctx, s, p, &coded));
+    // A state whose codes did not fit does not try again with the same time step, boundary type and
+    // coefficients: the attempt costs 65 to 80 us at 100^3, a staged step 50.
+    const size_t nC = (size_t)3 * nM * nM;
+    bool coded = !(s->noCodesHs == (int)h.hs && s->noCodesDt == p->dt && s->noCodesC.size() == nC &&
+                   !std::memcmp(s->noCodesC.data(), p->dTdtperdeltaT, 4 * nC));
+    if (coded) {
+      MCB_TRY(rows_build(ctx, s, p, &coded));
+      if (!coded && s->block) {  // (a view of the static scratch ends with its call and allocates nothing)
+        s->noCodesC.assign(p->dTdtperdeltaT, p->dTdtperdeltaT + nC);
+        s->noCodesDt = p->dt;
+        s->noCodesHs = (int)h.hs;
+      }
+    }
     if (coded) {
       k.rows = s;
       return MCB_OK;
