@@ -91,7 +91,6 @@ extern "C" mcb_status mcb_ctx_destroy(mcb_ctx *ctx) {
   for (auto &b : ctx->pool)
     if (b.ptr) cudaFree(b.ptr);
   if (ctx->heat) mcb_heat_state_destroy(ctx->heat);
-  if (ctx->heatLong) mcb_heat_state_destroy(ctx->heatLong);
   if (ctx->cancel_host) cudaFreeHost((void *)ctx->cancel_host);
   if (ctx->pin) cudaFreeHost(ctx->pin);
   if (ctx->ev0) cudaEventDestroy(ctx->ev0);

@@ -453,25 +453,40 @@ void free_state_buffers(mcb_heat_state *s) {
   s->sens = s->sIdx = nullptr;
   s->sensCap = 0;
   s->sCap = 0;
-  s->streamed = s->rowsOnly = false;
+  s->blockBytes = 0;
+  s->streamed = s->rowsOnly = s->either = false;
 }
 
 // The state's one allocation: its own, or its slot of the context's pool.
 mcb_status state_block(mcb_ctx *ctx, mcb_heat_state *s, size_t need) {
-  if (s->slot >= 0) return pool_get(ctx, s->slot, need, &s->block);
-  MCB_CUDA(ctx, cudaMalloc(&s->block, need));
+  if (s->slot >= 0) MCB_TRY(pool_get(ctx, s->slot, need, &s->block));
+  else MCB_CUDA(ctx, cudaMalloc(&s->block, need));
+  s->blockBytes = need;
   return MCB_OK;
 }
+
+constexpr size_t piece(size_t bytes) { return (bytes + 255) & ~(size_t)255; }
+
+// Pieces of a block, 256-byte aligned; from nullptr they are only counted.
+struct Carve {
+  char *cur;
+  size_t used = 0;
+  void *operator()(size_t bytes) {
+    char *q = cur;
+    if (cur) cur += piece(bytes);
+    used += piece(bytes);
+    return q;
+  }
+};
 
 // Streamed state (heat_stream.cu) for p's grid in one allocation, with its TMA descriptors.
 mcb_status stream_alloc(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *p, bool damage, bool rows = true) {
   free_state_buffers(s);
-  size_t need = 0;
+  Carve count{nullptr};
   mcb_heat_state probe{};
-  stream_carve([&](size_t b) { need += (b + 255) & ~(size_t)255; return (void *)nullptr; }, &probe, p, damage, true, rows);
-  MCB_TRY(state_block(ctx, s, need));
-  char *cur = (char *)s->block;
-  stream_carve([&](size_t b) { char *q = cur; cur += (b + 255) & ~(size_t)255; return (void *)q; }, s, p, damage, true, rows);
+  stream_carve(std::ref(count), &probe, p, damage, true, rows);
+  MCB_TRY(state_block(ctx, s, count.used));
+  stream_carve(Carve{(char *)s->block}, s, p, damage, true, rows);
   s->streamed = true;
   s->nx = p->nx;
   s->ny = p->ny;
@@ -479,8 +494,6 @@ mcb_status stream_alloc(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *
   s->nM = p->nM;
   s->L = (long long)p->nx * p->ny * p->nz;
   s->damage = damage;
-  s->rowsOnly = !stream_supported(p->nx, p->ny, p->nz);
-  if (s->rowsOnly) return MCB_OK;  // no TMA-staged passes
   s->maps = new StreamMaps();
   return stream_maps(ctx, s);
 }
@@ -516,28 +529,15 @@ bool state_fits(const mcb_heat_state *s, const mcb_heat_params *p, bool damage, 
          s->damage == damage;
 }
 
-mcb_status state_alloc(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *p, bool damage) {
+// Buffers of the factored state, carved by `take`, and its shape. The factorisation, which every time step and
+// boundary type forms anew, comes last (state_to_factored).
+void factored_carve(const std::function<void *(size_t)> &take, mcb_heat_state *s, const mcb_heat_params *p, bool damage) {
   const long long L = (long long)p->nx * p->ny * p->nz;
   const int nM = p->nM;
-  const size_t need = 4 * L * 3 /*T A Q*/ + 4 * (size_t)std::max<long long>(L, nM) /*stage*/ + 12 * L /*ib*/ +
-                      24 * L /*fb*/ + L /*nb*/ + 4 * L /*Sz*/ + (damage ? 8 * L : 0) + L + 12 * (size_t)nM * nM +
-                      24 * (size_t)nM /*logA E dmg*/ + 4 * (size_t)nM + 64 + 25 * 256;
-  free_state_buffers(s);
-  MCB_TRY(state_block(ctx, s, need));
-  char *cur = (char *)s->block;
-  auto take = [&](size_t bytes) {
-    char *q = cur;
-    cur += (bytes + 255) & ~(size_t)255;
-    return (void *)q;
-  };
   s->T = (float *)take(4 * L);
   s->A = (float *)take(4 * L);
   s->Q = (float *)take(4 * L);
   s->stage = (float *)take(4 * (size_t)std::max<long long>(L, nM));
-  s->ib = (float *)take(12 * L);
-  s->fb = (float2 *)take(24 * L);
-  s->nb = (uint8_t *)take(L);
-  s->Sz = (float *)take(4 * L);
   s->Om = damage ? (float *)take(4 * L) : nullptr;
   s->dOm = damage ? (float *)take(4 * L) : nullptr;
   s->M = (uint8_t *)take(L);
@@ -547,13 +547,64 @@ mcb_status state_alloc(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *p
   s->dmg = (float2 *)take(8 * (size_t)nM);
   s->maxEnc = (unsigned int *)take(4 * (size_t)nM);
   s->step = (int *)take(16);
+  s->ib = (float *)take(12 * L);
+  s->fb = (float2 *)take(24 * L);
+  s->nb = (uint8_t *)take(L);
+  s->Sz = (float *)take(4 * L);
   s->nx = p->nx;
   s->ny = p->ny;
   s->nz = p->nz;
   s->nM = nM;
   s->L = L;
   s->damage = damage;
+  s->streamed = s->rowsOnly = false;
+  s->factoredDt = -1.0;
   s->tw = std::min(yz_tile_width(p->ny), yz_tile_width(p->nz));
+}
+
+mcb_status state_alloc(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *p, bool damage) {
+  free_state_buffers(s);
+  Carve count{nullptr};
+  mcb_heat_state probe{};
+  factored_carve(std::ref(count), &probe, p, damage);
+  MCB_TRY(state_block(ctx, s, count.used));
+  factored_carve(Carve{(char *)s->block}, s, p, damage);
+  return MCB_OK;
+}
+
+// Grids with an axis over 512 that the coded passes take: streamed while their row codes fit, else factored.
+bool either_supported(const mcb_heat_params *p) {
+  return !stream_supported(p->nx, p->ny, p->nz) && rows_supported(p->nx, p->ny, p->nz);
+}
+
+// Lays the state out in its block, streamed or factored.
+void either_layout(mcb_heat_state *s, const mcb_heat_params *p, bool damage, bool streamed) {
+  if (streamed) {
+    stream_carve(Carve{(char *)s->block}, s, p, damage, true, true);
+    s->nx = p->nx;
+    s->ny = p->ny;
+    s->nz = p->nz;
+    s->nM = p->nM;
+    s->L = (long long)p->nx * p->ny * p->nz;
+    s->damage = damage;
+    s->streamed = s->rowsOnly = true;
+  } else {
+    factored_carve(Carve{(char *)s->block}, s, p, damage);
+  }
+}
+
+// A block for both layouts. It is as large as a factored state's (66 bytes per voxel; the streamed layout
+// takes 30 of the x-padded grid): only very short padded rows need more, as the temperatures and the damage
+// wait behind the streamed layout while one replaces the other (state_to_factored).
+mcb_status either_alloc(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *p, bool damage) {
+  free_state_buffers(s);
+  Carve streamed{nullptr}, factored{nullptr};
+  mcb_heat_state probe{};
+  stream_carve(std::ref(streamed), &probe, p, damage, true, true);
+  factored_carve(std::ref(factored), &probe, p, damage);
+  MCB_TRY(state_block(ctx, s, std::max(factored.used, streamed.used + 2 * piece(4 * (size_t)probe.L))));
+  s->either = true;
+  either_layout(s, p, damage, true);
   return MCB_OK;
 }
 
@@ -590,25 +641,17 @@ mcb_status state_upload(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *
   return state_upload_tables(ctx, s, p);
 }
 
-// A rowsOnly state whose row coefficients no longer fit the code tables (another dt or boundary type)
-// goes on as a factored one: T, the base and Omega stay on the device.
+// A rowsOnly state whose row coefficients do not fit the code tables (with this dt and boundary type) goes on
+// as a factored one in the same block: T and Omega wait at its end, where the factorisation will be.
 mcb_status state_to_factored(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *p) {
-  mcb_heat_state f;
-  f.ctx = ctx;
-  MCB_TRY(state_alloc(ctx, &f, p, s->damage));
-  f.base = s->base;
-  stream_dense_copy(ctx, s, f.T, ctx->stream);
-  mcb_status rc = MCB_OK;
-  if (s->damage && cudaMemcpyAsync(f.Om, s->Om, 4 * s->L, cudaMemcpyDeviceToDevice, ctx->stream) != cudaSuccess)
-    rc = set_error(ctx, MCB_ECUDA, "copy of the damage state failed");
-  if (rc == MCB_OK) rc = state_upload_tables(ctx, &f, p);
-  if (rc != MCB_OK) {
-    free_state_buffers(&f);
-    return rc;
-  }
-  free_state_buffers(s);
-  *s = f;
-  return MCB_OK;
+  const size_t grid = 4 * (size_t)s->L;
+  float *T = (float *)((char *)s->block + s->blockBytes - 2 * piece(grid)), *Om = T + piece(grid) / 4;
+  stream_dense_copy(ctx, s, T, ctx->stream);
+  if (s->damage) MCB_CUDA(ctx, cudaMemcpyAsync(Om, s->Om, grid, cudaMemcpyDeviceToDevice, ctx->stream));
+  either_layout(s, p, s->damage, false);
+  MCB_CUDA(ctx, cudaMemcpyAsync(s->T, T, grid, cudaMemcpyDeviceToDevice, ctx->stream));
+  if (s->damage) MCB_CUDA(ctx, cudaMemcpyAsync(s->Om, Om, grid, cudaMemcpyDeviceToDevice, ctx->stream));
+  return state_upload_tables(ctx, s, p);
 }
 
 HeatDev make_dev(const mcb_heat_state *s, const mcb_heat_params *p) {
@@ -758,24 +801,34 @@ extern "C" mcb_status mcb_heat_forward(mcb_ctx *ctx, const mcb_heat_params *p, f
     s->ctx = ctx;
     ctx->heat = s;
   }
-  if (stream_supported(p->nx, p->ny, p->nz) || rows_supported(p->nx, p->ny, p->nz)) {
+  const long long L = (long long)p->nx * p->ny * p->nz;
+  if (stream_supported(p->nx, p->ny, p->nz)) {
     if (!state_fits(s, p, damage, true)) MCB_TRY(stream_alloc(ctx, s, p, damage));
-    MCB_TRY(stream_upload(ctx, s, p, T, Omega, heat_mean(T, (long long)p->nx * p->ny * p->nz)));
+    MCB_TRY(stream_upload(ctx, s, p, T, Omega, heat_mean(T, L)));
     if (p->lightsOn) MCB_TRY(stream_upload_q(ctx, s, p->dTdt_abs));
     MCB_TRY(sensor_buffers(ctx, s, p));
-    bool fits = true;
-    MCB_TRY(stream_step(ctx, s, p, s->sens, sensorTemps, maxMediaTemps, true, &fits));
-    if (fits) return stream_download(ctx, s, T, Omega);
-    // a long grid of many media: the factored stepper, on a state of its own (the streamed one stays
-    // for the next call)
-    if (!ctx->heatLong) {
-      ctx->heatLong = new mcb_heat_state();
-      ctx->heatLong->ctx = ctx;
-    }
-    s = ctx->heatLong;
+    MCB_TRY(stream_step(ctx, s, p, s->sens, sensorTemps, maxMediaTemps, true));
+    return stream_download(ctx, s, T, Omega);
   }
-  if (!state_fits(s, p, damage, false)) MCB_TRY(state_alloc(ctx, s, p, damage));
-  MCB_TRY(state_upload(ctx, s, p, T, Omega, heat_mean(T, s->L)));
+  if (either_supported(p)) {
+    // the codes first, which need the geometry only; where they do not fit, the grids go to the factored layout
+    if (s->either && state_fits(s, p, damage, s->streamed)) either_layout(s, p, damage, true);
+    else MCB_TRY(either_alloc(ctx, s, p, damage));
+    MCB_TRY(stream_upload_media(ctx, s, p));
+    bool fits = false;
+    MCB_TRY(stream_codes(ctx, s, p, &fits));
+    if (fits) {
+      MCB_TRY(stream_upload_grids(ctx, s, T, Omega, heat_mean(T, L)));
+      if (p->lightsOn) MCB_TRY(stream_upload_q(ctx, s, p->dTdt_abs));
+      MCB_TRY(sensor_buffers(ctx, s, p));
+      MCB_TRY(stream_step(ctx, s, p, s->sens, sensorTemps, maxMediaTemps, true, nullptr, true));
+      return stream_download(ctx, s, T, Omega);
+    }
+    either_layout(s, p, damage, false);
+  } else if (!state_fits(s, p, damage, false)) {
+    MCB_TRY(state_alloc(ctx, s, p, damage));
+  }
+  MCB_TRY(state_upload(ctx, s, p, T, Omega, heat_mean(T, L)));
   MCB_TRY(state_step(ctx, s, p, sensorTemps, maxMediaTemps));
   return state_download(ctx, s, T, Omega);
 }
@@ -790,8 +843,9 @@ extern "C" mcb_status mcb_heat_state_create(mcb_ctx *ctx, const mcb_heat_params 
   mcb_heat_state *s = new mcb_heat_state();
   s->ctx = ctx;
   mcb_status st;
-  if (stream_supported(p->nx, p->ny, p->nz) || rows_supported(p->nx, p->ny, p->nz)) {
-    st = stream_alloc(ctx, s, p, Omega != nullptr);
+  const bool either = either_supported(p);
+  if (either || stream_supported(p->nx, p->ny, p->nz)) {
+    st = either ? either_alloc(ctx, s, p, Omega != nullptr) : stream_alloc(ctx, s, p, Omega != nullptr);
     if (st == MCB_OK) st = stream_upload(ctx, s, p, T, Omega, heat_mean(T, (long long)p->nx * p->ny * p->nz));
     if (st == MCB_OK && p->lightsOn) st = stream_upload_q(ctx, s, p->dTdt_abs);
   } else {

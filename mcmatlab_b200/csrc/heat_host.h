@@ -32,6 +32,7 @@ struct StreamMaps {
 struct mcb_heat_state {
   bool streamed = false;
   bool rowsOnly = false;  // streamed, with an axis over 512: coded-row passes only (no TMA-staged ones)
+  bool either = false;    // the block holds the streamed layout or the factored one (such a grid)
   mcb::StreamShape shape;
   mcb::StreamMaps *maps = nullptr;
   uint8_t *code = nullptr;
@@ -73,6 +74,7 @@ struct mcb_heat_state {
   long long sensCap = 0;
   int sCap = 0;
   void *block = nullptr;
+  size_t blockBytes = 0;
   int slot = -1;  // >= 0: the block is this slot of the context's buffer pool, not the state's own
 };
 
@@ -127,12 +129,18 @@ int stream_warmup(const float *c, float hdt, int nM);
 void stream_carve(const std::function<void *(size_t)> &take, mcb_heat_state *s, const mcb_heat_params *p, bool damage,
                   bool withQ, bool withRows);
 mcb_status stream_maps(mcb_ctx *ctx, mcb_heat_state *s);
+// stream_upload: the geometry (stream_upload_media), then T and Omega (stream_upload_grids).
+mcb_status stream_upload_media(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *p);
+mcb_status stream_upload_grids(mcb_ctx *ctx, mcb_heat_state *s, const float *T, const float *Omega, double base);
 mcb_status stream_upload(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *p, const float *T, const float *Omega,
                          double base);
+// Row codes of a rowsOnly state that holds its media; *fits false: more row coefficients than the tables hold.
+mcb_status stream_codes(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *p, bool *fits);
 mcb_status stream_upload_q(mcb_ctx *ctx, mcb_heat_state *s, const float *Q);
-// *fits false (nothing stepped): a rowsOnly state whose row coefficients do not fit the code tables.
+// *fits false (nothing stepped): a rowsOnly state whose row coefficients do not fit the code tables. coded:
+// stream_codes has formed this call's codes.
 mcb_status stream_step(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *p, double *sens, double *sensorTemps,
-                       float *maxMediaTemps, bool graphs, bool *fits = nullptr);
+                       float *maxMediaTemps, bool graphs, bool *fits = nullptr, bool coded = false);
 mcb_status stream_download(mcb_ctx *ctx, mcb_heat_state *s, float *T, float *Omega);
 // T of a streamed state (pitched deviations) into a dense array of deviations, and back;
 // asynchronous.

@@ -1245,32 +1245,46 @@ void stream_carve(const std::function<void *(size_t)> &take, mcb_heat_state *s, 
   if (withRows && rows_supported(S.nx, S.ny, S.nz)) rows_carve(take, s);
 }
 
-// Uploads M (pitched), the neighbourhood code, T (pitched deviations from `base`, the mean input
-// temperature) and Omega; clears the padding of every pitched grid.
-mcb_status stream_upload(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *p, const float *T, const float *Omega,
-                         double base) {
+// Uploads M (pitched) and forms the neighbourhood code; clears their padding.
+mcb_status stream_upload_media(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *p) {
   cudaStream_t st = ctx->stream;
   const StreamShape &S = s->shape;
   const long long L = (long long)S.nx * S.ny * S.nz;
   const Pitch P{S.nx, S.ny, S.nz, S.px};
   const int grid = ctx->num_sms * 8;
-  s->base = base;
-  MCB_CUDA(ctx, cudaMemsetAsync(s->T, 0, 4 * S.Lp, st));
-  MCB_CUDA(ctx, cudaMemsetAsync(s->A, 0, 4 * S.Lp, st));
-  if (s->Q) MCB_CUDA(ctx, cudaMemsetAsync(s->Q, 0, 4 * S.Lp, st));
   MCB_CUDA(ctx, cudaMemsetAsync(s->M, 0, S.Lp, st));
   MCB_CUDA(ctx, cudaMemsetAsync(s->code, 0, S.Lp, st));
   MCB_CUDA(ctx, cudaMemcpyAsync(s->stage, p->M, L, cudaMemcpyHostToDevice, st));
   to_pitched_u8_kernel<<<grid, 256, 0, st>>>((const uint8_t *)s->stage, s->M, P);
   code_kernel<<<grid, 256, 0, st>>>(s->M, s->code, P, p->heatBoundaryType != 0, L);
-  MCB_CUDA(ctx, cudaMemcpyAsync(s->stage, T, 4 * L, cudaMemcpyHostToDevice, st));
-  to_pitched_dev_kernel<<<grid, 256, 0, st>>>(s->stage, s->T, s->base, P);
-  if (s->Om && Omega) MCB_CUDA(ctx, cudaMemcpyAsync(s->Om, Omega, 4 * L, cudaMemcpyHostToDevice, st));
   MCB_CUDA(ctx, cudaGetLastError());
   s->codeHs = (int)(p->heatBoundaryType != 0);
   s->noCodesHs = -1;
+  return MCB_OK;
+}
+
+// Uploads T (pitched deviations from `base`, the mean input temperature) and Omega; clears the padding of
+// every other pitched grid.
+mcb_status stream_upload_grids(mcb_ctx *ctx, mcb_heat_state *s, const float *T, const float *Omega, double base) {
+  cudaStream_t st = ctx->stream;
+  const StreamShape &S = s->shape;
+  const long long L = (long long)S.nx * S.ny * S.nz;
+  s->base = base;
+  MCB_CUDA(ctx, cudaMemsetAsync(s->T, 0, 4 * S.Lp, st));
+  MCB_CUDA(ctx, cudaMemsetAsync(s->A, 0, 4 * S.Lp, st));
+  if (s->Q) MCB_CUDA(ctx, cudaMemsetAsync(s->Q, 0, 4 * S.Lp, st));
+  MCB_CUDA(ctx, cudaMemcpyAsync(s->stage, T, 4 * L, cudaMemcpyHostToDevice, st));
+  to_pitched_dev_kernel<<<ctx->num_sms * 8, 256, 0, st>>>(s->stage, s->T, s->base, Pitch{S.nx, S.ny, S.nz, S.px});
+  if (s->Om && Omega) MCB_CUDA(ctx, cudaMemcpyAsync(s->Om, Omega, 4 * L, cudaMemcpyHostToDevice, st));
+  MCB_CUDA(ctx, cudaGetLastError());
   s->qValid = false;
   return MCB_OK;
+}
+
+mcb_status stream_upload(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *p, const float *T, const float *Omega,
+                         double base) {
+  MCB_TRY(stream_upload_media(ctx, s, p));
+  return stream_upload_grids(ctx, s, T, Omega, base);
 }
 
 mcb_status stream_upload_q(mcb_ctx *ctx, mcb_heat_state *s, const float *Q) {
@@ -1296,12 +1310,29 @@ struct StreamStepper {
   bool ready = true;                     // false: a rowsOnly state without row codes
 };
 
+// Per-call tables on the device: H = dt/2 c with its diagonal and fixed points, and the damage exponents.
+static mcb_status stream_tables(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *p) {
+  const int nM = p->nM;
+  MCB_CUDA(ctx, cudaMemcpyAsync(s->H, p->dTdtperdeltaT, 12 * (size_t)nM * nM, cudaMemcpyHostToDevice, ctx->stream));
+  h_table_kernel<<<std::max(1, std::min(1024, (3 * nM * nM + 255) / 256)), 256, 0, ctx->stream>>>(s->H, s->Hd, (float)(p->dt / 2), nM);
+  float2 dmg[256];
+  heat_damage_table(p, s->base, dmg);
+  MCB_CUDA(ctx, cudaMemcpyAsync(s->dmg, dmg, 8 * (size_t)nM, cudaMemcpyHostToDevice, ctx->stream));
+  return MCB_OK;
+}
+
+mcb_status stream_codes(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *p, bool *fits) {
+  MCB_TRY(stream_tables(ctx, s, p));  // (the codes take the media that are damaged from it, not the base)
+  return rows_build(ctx, s, p, fits);
+}
+
 // Per-call set-up of the streamed stepper on a state: the per-call tables (H = dt/2 c in FP32, as
 // the stepper multiplies them, and its diagonal and fixed points, formed on the device; the
 // damage exponents about the base temperature; the pivot warm-up length), cleared maxima, step
 // counter and damage increments, kernel attributes and grids. `sens` is the device buffer of the
-// sensor history ([nS x (steps + 1)] doubles) or nullptr.
-mcb_status stream_setup(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *p, double *sens, StreamStepper *out) {
+// sensor history ([nS x (steps + 1)] doubles) or nullptr; ready: stream_codes has formed the row codes.
+mcb_status stream_setup(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *p, double *sens, StreamStepper *out,
+                        bool ready = false) {
   cudaStream_t st = ctx->stream;
   const StreamShape &S = s->shape;
   const long long L = (long long)S.nx * S.ny * S.nz;
@@ -1311,13 +1342,8 @@ mcb_status stream_setup(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *
     code_kernel<<<ctx->num_sms * 8, 256, 0, st>>>(s->M, s->code, Pitch{S.nx, S.ny, S.nz, S.px}, p->heatBoundaryType != 0, L);
     s->codeHs = (int)(p->heatBoundaryType != 0);
   }
-  const float hdt = (float)(p->dt / 2);
-  MCB_CUDA(ctx, cudaMemcpyAsync(s->H, p->dTdtperdeltaT, 12 * (size_t)nM * nM, cudaMemcpyHostToDevice, st));
-  h_table_kernel<<<std::max(1, std::min(1024, (3 * nM * nM + 255) / 256)), 256, 0, st>>>(s->H, s->Hd, hdt, nM);
-  float2 dmg[256];
-  heat_damage_table(p, s->base, dmg);
-  const int W = stream_warmup(p->dTdtperdeltaT, hdt, nM);
-  MCB_CUDA(ctx, cudaMemcpyAsync(s->dmg, dmg, 8 * (size_t)nM, cudaMemcpyHostToDevice, st));
+  MCB_TRY(stream_tables(ctx, s, p));
+  const int W = stream_warmup(p->dTdtperdeltaT, (float)(p->dt / 2), nM);
   MCB_CUDA(ctx, cudaMemsetAsync(s->maxEnc, 0, 4 * (size_t)nM, st));
   MCB_CUDA(ctx, cudaMemsetAsync(s->step, 0, 16, st));
   if (s->dOm) MCB_CUDA(ctx, cudaMemsetAsync(s->dOm, 0, 4 * (size_t)S.Lp, st));
@@ -1338,6 +1364,10 @@ mcb_status stream_setup(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *
   k.S = S;
   // The codes cost about three of the steps they speed up (100^3: 60 us against 20 saved per step,
   // 300x300x200: 0.45 ms against 0.17), so shorter calls take the staged passes.
+  if (ready) {
+    k.rows = s;
+    return MCB_OK;
+  }
   if (s->rowX && (s->rowsOnly || p->steps >= 4)) {
     // A state whose codes did not fit does not try again with the same time step, boundary type and
     // coefficients: the attempt costs 65 to 80 us at 100^3, a staged step 50.
@@ -1446,13 +1476,13 @@ void stream_pitched_indices(const mcb_heat_state *s, const int *dense, int *pitc
 // Runs p->steps steps on the device-resident streamed state. Sensor and maximum outputs go to
 // host memory; `sens` is the device buffer of the sensor history ([nS x (steps + 1)] doubles).
 mcb_status stream_step(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *p, double *sens, double *sensorTemps,
-                       float *maxMediaTemps, bool graphs, bool *fits) {
+                       float *maxMediaTemps, bool graphs, bool *fits, bool coded) {
   cudaStream_t st = ctx->stream;
   const StreamShape &S = s->shape;
   const long long L = (long long)S.nx * S.ny * S.nz, nt = p->steps;
   const int nM = p->nM, nS = p->nSensors;
   StreamStepper ks;
-  MCB_TRY(stream_setup(ctx, s, p, sens, &ks));
+  MCB_TRY(stream_setup(ctx, s, p, sens, &ks, coded));
   if (fits) *fits = ks.ready;
   if (!ks.ready) return MCB_OK;
   const StreamDev &h = ks.h;

@@ -29,7 +29,6 @@ struct mcb_ctx {
   std::vector<DevBuf> pool;             // indexed slots, grow-only
   int num_sms = 0;
   mcb_heat_state *heat = nullptr;  // state reused by mcb_heat_forward
-  mcb_heat_state *heatLong = nullptr;  // its factored state for long grids whose row codes do not fit
   void *pin = nullptr;             // kPinBytes of page-locked host memory: small results leave through it
   double lastKernelMs = 0.0;        // device time of the last stepping / transport loop
   // transport launch parameters: tuned per size class (mcb_mc_autotune, or read from the tuning

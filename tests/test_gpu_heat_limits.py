@@ -190,3 +190,68 @@ def test_state_whose_codes_fit_at_some_steps_only(oracle_lib):
     finally:
         st.close()
     assert np.max(np.abs(Tg - T) / np.abs(T)) <= 5e-5  # 1e-5 per call, as the stepper's other tests
+
+
+def test_long_state_whose_codes_fit_at_first(oracle_lib):
+    """The same on an axis over 512, where a state whose codes do not fit goes on as a factored one: with
+    its temperatures, and with its damage to the bit (no medium adds any here)."""
+    from mcmatlab_b200 import native
+    from oracle import orc
+    shape = (8, 9, 600)
+    case = voxelwise(shape, 2, 4)
+    O0 = np.asfortranarray(np.random.default_rng(5).random(shape).astype(np.float32))
+    none = np.zeros((2, 1))
+    calls = [dict(case["hp"], dt=dt, A=none, E=none) for dt in (1e-6, 2.0, 2.0, 1e-6)]
+    assert max(row_codes(calls[0])) <= 255 < max(row_codes(calls[1]))
+    T = case["T0"].astype(np.float64)
+    st = native.HeatState(case["T0"], O0, calls[0], *shape)
+    try:
+        for k, hp in enumerate(calls):
+            st.step(hp)
+            T, _, _, _ = orc.oracle_heat(T.astype(np.float32), None, hp, *shape)
+            Tg, Og = st.read()
+            assert np.max(np.abs(Tg - T) / np.abs(T)) <= 1e-5 * (k + 1)
+            np.testing.assert_array_equal(Og, O0)
+    finally:
+        st.close()
+
+
+def test_long_calls_in_turn_share_one_block(oracle_lib):
+    """Whole calls on one context, some with codes that fit and some without, with and without damage: each
+    equals the oracle, and what the context holds for them afterwards is one factored state (66 bytes per
+    voxel; the bound leaves room for the allocator's pages), not a streamed one beside it."""
+    import torch
+    from mcmatlab_b200 import abi, native
+    from oracle import orc
+    lib, fp = native.lib(), ctypes.POINTER(ctypes.c_float)
+    shape = (64, 60, 700)
+
+    def call(ctx, case, hp, damage):
+        hb = abi.HeatParamBuffers(*case["n"], hp)
+        T = np.ascontiguousarray(case["T0"].reshape(-1, order="F")).copy()
+        O = np.zeros(T.size, np.float32)
+        mx = np.zeros(hb.nM, np.float32)
+        st = lib.mcb_heat_forward(ctx, ctypes.byref(hb.params), T.ctypes.data_as(fp),
+                                  O.ctypes.data_as(fp) if damage else ctypes.cast(None, fp),
+                                  ctypes.cast(None, ctypes.POINTER(ctypes.c_double)), mx.ctypes.data_as(fp))
+        assert st == 0, lib.mcb_last_error(ctx).decode()
+        return T.reshape(case["n"], order="F"), O.reshape(case["n"], order="F")
+
+    ctx = ctypes.c_void_p()
+    assert lib.mcb_ctx_create(0, ctypes.byref(ctx)) == 0
+    try:
+        small, case = voxelwise((16, 8, 520), 2, 3), voxelwise(shape, 2, 3)
+        for dt in (1e-6, 2.0):  # loads the kernels
+            call(ctx, small, dict(small["hp"], dt=dt), True)
+        free = torch.cuda.mem_get_info(0)[0]
+        for dt, damage in ((2.0, True), (1e-6, True), (2.0, True), (1e-6, False), (2.0, False)):
+            hp = dict(case["hp"], dt=dt)
+            T, O = call(ctx, case, hp, damage)
+            To, Oo, _, _ = orc.oracle_heat(case["T0"], np.zeros(shape, np.float32) if damage else None, hp, *shape)
+            assert np.max(np.abs(T - To) / np.abs(To)) <= 1e-5
+            if damage:
+                assert np.max(np.abs(O - Oo)) <= 1e-4 * np.max(Oo)
+        held = free - torch.cuda.mem_get_info(0)[0]
+        assert held <= 72 * np.prod(shape) + (8 << 20), held / np.prod(shape)
+    finally:
+        lib.mcb_ctx_destroy(ctx)
