@@ -160,8 +160,8 @@ MCB_API mcb_status mcb_mc_normalize(mcb_ctx *ctx, const mcb_mc_model *model, con
 /* No counterpart in the reference, which sizes its launch with cudaOccupancyMaxPotentialBlockSize
  * (MCmatlab.c:641): the transport kernel's warp-grouping parameters. refillMin: a warp launches
  * new packets on its free lanes once at least this many lanes are free; scatterMin: packets whose
- * free path ran out wait until this many lanes of their warp are waiting before roulette and
- * scattering run (both 1..32). Results do not depend on them (each packet's random stream is
+ * free path ran out wait until this many of their warp's 32 lanes are waiting, or the same share of
+ * the lanes that still hold a packet, before roulette and scattering run (both 1..32). Results do not depend on them (each packet's random stream is
  * fixed); only the time does. */
 typedef struct mcb_mc_launch {
   int32_t refillMin, scatterMin;

@@ -45,7 +45,7 @@ struct KernelArgs {
   // Refill threshold: a warp re-launches free lanes only when at least this many are free (or
   // none is alive), so the divergent launch code runs once for a group of lanes.
   int refillMin;   // free lanes a warp waits for before launching new packets
-  int scatterMin;  // waiting lanes before roulette + scattering run
+  int scatterMin;  // waiting lanes of 32 alive before roulette + scattering run (the same share of fewer)
   int lanes;       // lanes of a warp that take packets (fewer where the packets do not fill the grid)
 };
 
@@ -340,15 +340,15 @@ __global__ void __launch_bounds__(256, GRAD ? 3 : 4) transport_kernel(KernelArgs
     // 4. scattering events in groups: a packet whose free path is used up waits (no sub-step)
     //    until enough lanes of its warp are waiting too, or no lane can take a sub-step, so the
     //    long scattering code runs with most lanes active. A packet's events and random draws do
-    //    not change, only when its warp performs them. The group size (a.scatterMin) is a launch
-    //    parameter of the autotuner, but at most a quarter of the lanes still alive: in a thinned-out
-    //    warp (few packets, the end of a run) waiting for a full group only adds latency (half of the
+    //    not change, only when its warp performs them. The group (a.scatterMin of 32 lanes) is a launch
+    //    parameter of the autotuner; a thinned-out warp (few packets, the end of a run) takes the same
+    //    share of the lanes still alive, as waiting for a full group only adds latency there (half of the
     //    lanes: 322 us on a 30^3 grid of 1e4 packets, a quarter 292, an eighth 289 but 5% more on full warps).
     {
       const bool want = P.alive && !(P.stepLeft > 0);
       const unsigned waiting = __ballot_sync(0xffffffffu, want);
       const unsigned stepping = __ballot_sync(0xffffffffu, P.alive && P.stepLeft > 0);
-      if (want && (__popc(waiting) >= min(a.scatterMin, (__popc(waiting | stepping) + 3) >> 2) || stepping == 0)) {
+      if (want && (__popc(waiting) >= (a.scatterMin * __popc(waiting | stepping) + 31) >> 5 || stepping == 0)) {
         if (P.weight < kThreshold) {
           if (rnd(P, *I) <= kChance) P.weight /= kChance;
           else P.alive = false;
@@ -950,14 +950,14 @@ int size_class(long long voxels, bool grad, bool batched) {
   return c + (grad ? 16 : 0) + (batched ? 32 : 0);
 }
 
-// The autotuner's override, else the class's tuned parameters, else the defaults: (12, 8) on the
-// 100^3 cube (5.07 ms for 1e6 packets, 5.16 at 16, 8) and (12, 12) for gradients; all pairs from (8, 8)
-// to (16, 12) lie within 2% of each other.
+// The autotuner's override, else the class's tuned parameters, else (12, 8). Of the autotuner's 16 pairs the
+// 100^3 cube (1e6 packets) takes 4.41 to 4.72 ms, 4.46 at (12, 8), and gradients on 256^3 17.7 to 19.5 ms, 18.8
+// at (12, 8): there the small refill groups are the faster ones, on smaller grids the larger.
 mcb_mc_launch launch_params(const mcb_ctx *ctx, int cls, bool grad) {
   if (ctx->force.refillMin > 0) return ctx->force;
   const auto it = ctx->tuned.find(cls);
   if (it != ctx->tuned.end()) return it->second;
-  return grad ? mcb_mc_launch{12, 12} : mcb_mc_launch{12, 8};
+  return mcb_mc_launch{12, 8};
 }
 
 mcb_status launch_transport(mcb_ctx *ctx, Arena &ar, const std::vector<Inst> &insts, bool openEnded,
