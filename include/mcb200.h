@@ -47,7 +47,10 @@ typedef enum {
 
 typedef struct mcb_ctx mcb_ctx;
 
-/* One context per device and caller thread; it owns device buffers reused across calls. */
+/* One context per device and caller thread. It owns device buffers that calls leave for later ones:
+ * each entry's largest work memory, the state of mcb_heat_forward's last grid (30 bytes per voxel, 66
+ * for grids with an axis over 512), the adjoint's work memory, and up to 512 MiB of the adjoint's
+ * states. mcb_ctx_destroy gives them back. */
 MCB_API mcb_status mcb_ctx_create(int device, mcb_ctx **out);
 MCB_API mcb_status mcb_ctx_destroy(mcb_ctx *ctx);
 MCB_API const char *mcb_last_error(const mcb_ctx *ctx);

@@ -30,8 +30,13 @@ mcb_status pool_get(mcb_ctx *ctx, int slot, size_t bytes, void **out) {
       b.ptr = nullptr;
       b.bytes = 0;
     }
-    const size_t want = bytes + bytes / 8;
+    size_t want = bytes + bytes / 8;
     cudaError_t e = cudaMalloc(&b.ptr, want);
+    if (e == cudaErrorMemoryAllocation) {  // without the room to grow
+      cudaGetLastError();
+      want = bytes;
+      e = cudaMalloc(&b.ptr, want);
+    }
     if (e != cudaSuccess) {
       cudaGetLastError();
       b.ptr = nullptr;
@@ -41,6 +46,13 @@ mcb_status pool_get(mcb_ctx *ctx, int slot, size_t bytes, void **out) {
   }
   *out = b.ptr;
   return MCB_OK;
+}
+
+void pool_free(mcb_ctx *ctx, int slot) {
+  if ((int)ctx->pool.size() <= slot || !ctx->pool[slot].ptr) return;
+  cudaStreamSynchronize(ctx->stream);
+  cudaFree(ctx->pool[slot].ptr);
+  ctx->pool[slot] = DevBuf{};
 }
 
 }  // namespace mcb

@@ -46,6 +46,9 @@ mcb_status set_error(mcb_ctx *ctx, mcb_status st, const char *fmt, ...);
 // Returns a device buffer for `slot` of at least `bytes` (contents undefined).
 mcb_status pool_get(mcb_ctx *ctx, int slot, size_t bytes, void **out);
 
+// Gives the buffer of `slot` back to the device.
+void pool_free(mcb_ctx *ctx, int slot);
+
 constexpr size_t kPinBytes = (size_t)1 << 20;
 
 // Index of the first of p[0..n) outside lo..hi, or -1. Whole blocks are judged by one maximum, which

@@ -255,3 +255,38 @@ def test_long_calls_in_turn_share_one_block(oracle_lib):
         assert held <= 72 * np.prod(shape) + (8 << 20), held / np.prod(shape)
     finally:
         lib.mcb_ctx_destroy(ctx)
+
+
+def test_adjoint_gives_large_states_back():
+    """After an adjoint on 8.4 million voxels the context holds its work memory (ten grids and the pool's eighth:
+    45 bytes per voxel) and not the two states beside it (another 90)."""
+    import torch
+    from mcmatlab_b200 import abi, native
+    lib, fp = native.lib(), ctypes.POINTER(ctypes.c_float)
+
+    def call(ctx, shape):
+        case = voxelwise(shape, 2, 2)
+        hb = abi.HeatParamBuffers(*shape, case["hp"])
+        T = np.ascontiguousarray(case["T0"].reshape(-1, order="F"))
+        w = np.zeros(T.size, np.float32)
+        w[T.size // 2:T.size // 2 + 9] = 1.0
+        obj, g = abi.mcb_heat_objective(), abi.mcb_heat_grad()
+        obj.damageWeight, obj.peakWeight = w.ctypes.data_as(fp), ctypes.cast(None, fp)
+        dT = np.zeros(T.size, np.float32)
+        g.dJ_dT0 = dT.ctypes.data_as(fp)
+        assert lib.mcb_heat_adjoint(ctx, ctypes.byref(hb.params), T.ctypes.data_as(fp), ctypes.byref(obj), 0, ctypes.byref(g)) == 0
+        return dT
+
+    ctx = ctypes.c_void_p()
+    assert lib.mcb_ctx_create(0, ctypes.byref(ctx)) == 0
+    try:
+        small = call(ctx, (30, 28, 24))
+        free = torch.cuda.mem_get_info(0)[0]
+        shape = (256, 256, 128)
+        big = call(ctx, shape)
+        held = free - torch.cuda.mem_get_info(0)[0]
+        assert held <= 50 * np.prod(shape), held / np.prod(shape)
+        np.testing.assert_allclose(call(ctx, shape), big, rtol=1e-4, atol=1e-6 * np.abs(big).max())
+        np.testing.assert_allclose(call(ctx, (30, 28, 24)), small, rtol=1e-4, atol=1e-6 * np.abs(small).max())
+    finally:
+        lib.mcb_ctx_destroy(ctx)
