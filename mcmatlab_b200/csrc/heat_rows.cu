@@ -1,7 +1,8 @@
 // Coded-row passes of the streamed DG-ADI stepper for sm_100a: the stepping path of
 // mcb_heat_forward and mcb_heat_state_* (replacing
-// +MCmatlab/src/finiteElementHeatPropagator.c:249-647) on every grid whose line coefficients fit
-// the code tables below; other calls step with the TMA-staged passes of heat_stream.cu.
+// +MCmatlab/src/finiteElementHeatPropagator.c:249-647) on grids of up to 796 voxels along x and 1024 along
+// y and z whose line coefficients fit the code tables below; other calls step with the TMA-staged passes of
+// heat_stream.cu or, on axes over 512, with the factored stepper of heat_adi.cu.
 //
 // The step is taken in its increments, which is the same algebra as substeps 1a..3b
 // (X, Y, Z = I - dt/2 D_x, D_y, D_z):
@@ -17,9 +18,12 @@
 // (pivots in FP64, rounded once), collects the triples in a 255-entry hash table per direction and
 // stores one byte per row. The passes look the byte up in shared memory, so all rows of all lines
 // run one branch-free path with no pivot recurrence, no medium lookup and no interface case. The
-// four y and z face coefficients of the explicit stencil are coded the same way. Where a
-// direction has more than 255 triples (media varying voxel by voxel), the call steps with the
-// passes of heat_stream.cu.
+// four y and z face coefficients of the explicit stencil are coded the same way.
+// Where a direction has more than 255 of them, the call steps with the other passes. Every neighbourhood
+// of media adds the pivots of its convergence, so the count grows with the inclusions and with the time
+// step. On 100^3 voxels, the most along an axis: layers and one inclusion 32 (95 at 15 times the explicit limit),
+// ten inclusions of 4 media 126 (453), twenty of 6 media 302 (1211), thirty of 8 media 372, one medium in 40
+// smooth sub-media 1028; media varying by voxel fit with two media at most.
 //
 // Layout of the passes: a lane owns K = 16 (or 32) consecutive rows of one line in registers, the
 // 32 lanes of a warp 32 lines, the warps of a block the chunks of the same 32 lines; its K codes
@@ -37,6 +41,10 @@
 // stencil) and by their loads' latency at two blocks per SM. The passes before spent 126 to 235
 // thread instructions per voxel on pivot recurrences, interface tests and per-tile set-up; these
 // spend 43 (Y), 86 (Z) and 107 (X) at 100^3.
+// Spills (bytes stored / loaded): X up to 128 rows and from 321 to 512 none, 129 to 320 32 / 36 (48 registers, for
+// two blocks per SM), over 512 468 / 564; Y up to 512 rows none but 24 / 24 at 209 to 320, to 640 44 / 44, to
+// 1024 492 / 636; Z 16 / 16 up to 128, 52 / 80 to 208, none to 320, 108 / 164 to 512, 420 / 576 to 640,
+// 812 / 1100 to 1024.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -127,7 +135,7 @@ __device__ __forceinline__ int probe_code(unsigned long long *keys, float4 *tab,
 // of a warp mostly hold the same rows, and all warps of the first wave look for the same few keys at once).
 // The cache has 256 words of 56 bits of the hash, which with its 8-bit index is all of it and so the key (the
 // multiplier is odd), and the code; a word is read and written whole. 100^3 voxels: the coding kernel 71 -> 66 us
-// with layers and one inclusion, 95 -> 81 with ten inclusions of 4 media. (A function of its own: inlined at
+// with layers and one inclusion, 95 -> 81 with ten inclusions of 4 media (at three blocks per SM). (A function of its own: inlined at
 // every row of the unrolled walks it takes their registers.)
 __device__ __noinline__ int find_code(volatile unsigned long long *cache, unsigned long long *keys, float4 *tab, int *med, int *over,
                                       unsigned long long key, float4 e, int medium) {
@@ -238,8 +246,10 @@ __device__ __forceinline__ void line_codes(const RowBuild &b, const uint8_t *can
   }
 }
 
-// Codes of every row (blockIdx.y: 0 x-lines, 1 y columns, 2 z columns, 3 the y and z faces).
-__global__ void __launch_bounds__(128) rows_code_kernel(const RowBuild b) {
+// Codes of every row (blockIdx.y: 0 x-lines, 1 y columns, 2 z columns, 3 the y and z faces). Four blocks per SM:
+// the walks wait for loads and for the pivots' divisions (three at 140 registers 737 us at 300x300x200, four
+// 623, 62 at 100^3).
+__global__ void __launch_bounds__(128, 4) rows_code_kernel(const RowBuild b) {
   __shared__ uint8_t canon[256];
   __shared__ unsigned long long cache[256];  // find_code
   for (int k = threadIdx.x; k < 256; k += blockDim.x) {

@@ -2,9 +2,10 @@
 // mcb_heat_state_* (replacing +MCmatlab/src/finiteElementHeatPropagator.c:688-821) for grids
 // whose axes are at most 512 voxels long: state, set-up and host side, and the TMA-staged passes.
 // Calls step with the coded-row passes of heat_rows.cu where their row codes fit (2.0x the
-// TMA-staged passes at 100^3, 1.85x at 300x300x200); the TMA-staged passes step the others: media
-// that vary voxel by voxel (more than 255 row coefficients along an axis), calls of
-// mcb_heat_forward_static whose scratch has no room for the codes, and the adjoint's forward sweeps.
+// TMA-staged passes at 100^3, 1.85x at 300x300x200); the TMA-staged passes step the others: geometries with
+// more than 255 row coefficients along an axis (dozens of inclusions, many sub-media; heat_rows.cu gives
+// counts), calls of fewer than four steps, calls of mcb_heat_forward_static whose scratch has no room for
+// the codes, and the adjoint's forward sweeps.
 //
 // One time step of the reference is six grid passes (substep1a..3b, :249-647). Here it is three
 // streaming passes, one per direction, and nothing per voxel is stored besides the state:
@@ -1362,8 +1363,9 @@ mcb_status stream_setup(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *
   s->lastW = h.W;
 
   k.S = S;
-  // The codes cost about three of the steps they speed up (100^3: 60 us against 20 saved per step,
-  // 300x300x200: 0.45 ms against 0.17), so shorter calls take the staged passes.
+  // The codes cost about three of the steps they speed up (100^3: 62 us against 20 saved per step, 80 with ten
+  // inclusions; 300x300x200: 0.62 ms against 0.17), so shorter calls take the staged passes. A call
+  // whose codes do not fit finds out in 65 to 80 us.
   if (ready) {
     k.rows = s;
     return MCB_OK;

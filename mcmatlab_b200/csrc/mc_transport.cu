@@ -952,7 +952,7 @@ int size_class(long long voxels, bool grad, bool batched) {
 
 // The autotuner's override, else the class's tuned parameters, else (12, 8). Of the autotuner's 16 pairs the
 // 100^3 cube (1e6 packets) takes 4.41 to 4.72 ms, 4.46 at (12, 8), and gradients on 256^3 17.7 to 19.5 ms, 18.8
-// at (12, 8): there the small refill groups are the faster ones, on smaller grids the larger.
+// at (12, 8): the small refill groups are the faster ones there.
 mcb_mc_launch launch_params(const mcb_ctx *ctx, int cls, bool grad) {
   if (ctx->force.refillMin > 0) return ctx->force;
   const auto it = ctx->tuned.find(cls);
