@@ -46,7 +46,7 @@ sys.path.insert(0, ROOT)
 from mcmatlab_b200 import configs, mexargs, prep  # noqa: E402
 
 METRIC = "photon packets/s, heat voxel-updates/s on 1 B200; batched+adjoint vs plain"
-HEAT_STEP_DRAM_BYTES = 27.4e6
+HEAT_STEP_DRAM_BYTES = 27.6e6
 N_GRID = 100
 MC_PACKETS = 1_000_000
 
@@ -248,7 +248,8 @@ def run_ours(args):
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
                      "peak_source": src,
                      # DRAM bytes of one DG-ADI step (X + Y + Z pass) from a cold-cache ncu capture of
-                     # this workload (reads; the writes stay in L2); in the timed loop the grid is
+                     # this workload (reads; the writes stay in L2) in
+                     # profiles/heat_rows_passes_100cube_300x300x200.md; in the timed loop the grid is
                      # L2-resident
                      "traffic": HEAT_STEP_DRAM_BYTES, "traffic_note": "ncu cold-cache capture, bytes per DG-ADI step",
                      "algorithmic_bytes_per_voxel_update": bytes_per_update,
