@@ -88,6 +88,7 @@ struct RowBuild {
   uint4 *x, *y, *z;
   int GX, GY, GZ;
   uint8_t canon[256];  // smallest medium with the same couplings
+  unsigned int first[4];  // first block of each job of rows_code_kernel
 };
 
 __global__ void rows_init_kernel(unsigned long long *keys, float4 *tab, int *med, int *over) {
@@ -246,19 +247,22 @@ __device__ __forceinline__ void line_codes(const RowBuild &b, const uint8_t *can
   }
 }
 
-// Codes of every row (blockIdx.y: 0 x-lines, 1 y columns, 2 z columns, 3 the y and z faces). Four blocks per SM:
-// the walks wait for loads and for the pivots' divisions (three at 140 registers 737 us at 300x300x200, four
-// 623, 62 at 100^3).
+// Codes of every row: the blocks from b.first[job] on take x-lines (job 0), y columns (1), z columns (2) and the
+// y and z faces (3). Four blocks per SM: the walks wait for loads and for the pivots' divisions (three at 140
+// registers 737 us at 300x300x200, four 623), and no block is launched for nothing (with a row of blocks per
+// job, each as long as the longest, 623 us; as now 432, and 62 -> 51 at 100^3). A block that starts after a table
+// has overflowed ends at once: what such a call pays is 50 to 80 us at 100^3, 110 to 300 at 300x300x200.
 __global__ void __launch_bounds__(128, 4) rows_code_kernel(const RowBuild b) {
   __shared__ uint8_t canon[256];
   __shared__ unsigned long long cache[256];  // find_code
+  if (__syncthreads_or(threadIdx.x == 0 && rows_over(b))) return;
   for (int k = threadIdx.x; k < 256; k += blockDim.x) {
     canon[k] = b.canon[k];
     cache[k] = 0ull;
   }
   __syncthreads();
-  const int job = blockIdx.y;
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const int job = blockIdx.x < b.first[2] ? (blockIdx.x < b.first[1] ? 0 : 1) : (blockIdx.x < b.first[3] ? 2 : 3);
+  const long long t = (blockIdx.x - b.first[job]) * (long long)blockDim.x + threadIdx.x;
   if (job == 3) {
     const int quads = b.px / 4;
     if (t >= (long long)b.ny * b.nz * quads) return;
@@ -864,8 +868,13 @@ mcb_status rows_build(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *p,
     }
   }
   rows_init_kernel<<<4, kCodes, 0, st>>>(b.keys, b.tab, b.med, b.over);
-  const long long most = std::max({(long long)S.ny * S.nz * (S.px / 4), (long long)S.px * S.nz, (long long)S.px * S.ny, (long long)S.ny * S.nz + 31});
-  rows_code_kernel<<<dim3((unsigned)((most + 127) / 128), 4), 128, 0, st>>>(b);
+  const long long items[4] = {(long long)S.ny * S.nz + 31, (long long)S.px * S.nz, (long long)S.px * S.ny, (long long)S.ny * S.nz * (S.px / 4)};
+  unsigned int blocks = 0;
+  for (int job = 0; job < 4; job++) {
+    b.first[job] = blocks;
+    blocks += (unsigned int)((items[job] + 127) / 128);
+  }
+  rows_code_kernel<<<blocks, 128, 0, st>>>(b);
   MCB_CUDA(ctx, cudaGetLastError());
   MCB_TRY(x_kernel(S.nx, [&](auto kern) { return smem_allow(ctx, (const void *)kern, x_tile(S.nx)); }));
   int over = 0;

@@ -1363,16 +1363,16 @@ mcb_status stream_setup(mcb_ctx *ctx, mcb_heat_state *s, const mcb_heat_params *
   s->lastW = h.W;
 
   k.S = S;
-  // The codes cost about three of the steps they speed up (100^3: 62 us against 20 saved per step, 80 with ten
-  // inclusions; 300x300x200: 0.62 ms against 0.17), so shorter calls take the staged passes. A call
-  // whose codes do not fit finds out in 65 to 80 us.
+  // The codes cost about three of the steps they speed up (100^3: 51 us against 20 saved per step, 70 with ten
+  // inclusions; 300x300x200: 0.43 ms against 0.17), so shorter calls take the staged passes. A call
+  // whose codes do not fit finds out in 50 to 80 us, 110 to 300 at 300x300x200.
   if (ready) {
     k.rows = s;
     return MCB_OK;
   }
   if (s->rowX && (s->rowsOnly || p->steps >= 4)) {
     // A state whose codes did not fit does not try again with the same time step, boundary type and
-    // coefficients: the attempt costs 65 to 80 us at 100^3, a staged step 50.
+    // coefficients: the attempt costs 50 to 80 us at 100^3, a staged step 50.
     const size_t nC = (size_t)3 * nM * nM;
     bool coded = !(s->noCodesHs == (int)h.hs && s->noCodesDt == p->dt && s->noCodesC.size() == nC &&
                    !std::memcmp(s->noCodesC.data(), p->dTdtperdeltaT, 4 * nC));
